@@ -436,6 +436,44 @@ int b200_topk_softmax(const void* gating_output, int dtype, int64_t row_stride, 
                       void* stream);
 
 /*
+ * One block-FP8 linear, start to finish: out[M,N] = quantise(x)[M,K] * w[N,K]^T (+ bias), the call sequence of
+ * Fp8LinearMethod.apply (python/sglang/srt/layers/quantization/fp8.py:441-488).  x, bias [N] (or NULL) and out share
+ * `dtype` (bf16 / fp16); bias is added to the rounded product.  K % 128 == 0.
+ * scale_mode 0: fp32 scales; 1: power-of-two activation scales; 2: weight scales are powers of two as well.
+ * Everything in between lives in `workspace` (b200_fp8_linear_workspace_bytes bytes, 16-byte aligned), which may be
+ * reused by the next call on the same stream.  b200_sm_count: SMs the persistent kernels use on the current device.
+ */
+size_t b200_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K, int scale_mode);
+int b200_fp8_linear(const void* x, int dtype, const void* w, int64_t ldw, const float* ws, int64_t ws_stride_n,
+                    int64_t ws_stride_g, const void* bias, void* out, int64_t ldo, int64_t M, int64_t N, int64_t K,
+                    int scale_mode, void* workspace, size_t workspace_bytes, void* stream);
+int b200_sm_count(void);
+
+/*
+ * The fused expert layer, start to finish (cutlass_fused_experts_fp8, python/sglang/srt/layers/moe/cutlass_moe.py:29-222):
+ * x [m,k] -> out [m,k] in `dtype`; w13 [E,2n,k], w2 [E,k,n] e4m3 contiguous with block scales [E,2n/128,k/128] and
+ * [E,k/128,n/128]; topk_weights fp32 (each rounded to `dtype` before the weighted sum) and topk_ids int32 [m,topk], ids
+ * < 0 contribute nothing.  scale_ue8m0 != 0: power-of-two scales throughout (the weights' too).  expert_offsets [E+1]
+ * and problem_sizes1/2 [E,3] receive the routing tables when not NULL.
+ */
+size_t b200_fused_experts_fp8_workspace_bytes(int64_t m, int64_t k, int64_t n, int topk, int num_experts, int scale_ue8m0);
+int b200_fused_experts_fp8(const void* x, int dtype, const void* w13, const void* w2, const float* w13_scale,
+                           const float* w2_scale, const float* topk_weights, const int32_t* topk_ids, int64_t m, int64_t k,
+                           int64_t n, int topk, int num_experts, int32_t* expert_offsets, int32_t* problem_sizes1,
+                           int32_t* problem_sizes2, void* out, int scale_ue8m0, void* workspace, size_t workspace_bytes,
+                           void* stream);
+
+/*
+ * Dense MLP, first half, on the block-scaling path: b200_fp8_blockwise_scaled_grouped_mm_pow2_silu_quant for ONE problem
+ * of M rows, without a problem table in device memory.  b [2N,K], gate rows first.
+ */
+int b200_fp8_gate_up_silu_quant_pow2(const void* a, int64_t lda, const void* b, int64_t ldb, const uint32_t* sa_packed,
+                                     int64_t sa_stride_m, int64_t sa_stride_pack, const float* sb_pow2, int64_t sb_stride_n,
+                                     int64_t sb_stride_g, void* out_q, int64_t ldq, uint32_t* out_s,
+                                     int64_t out_s_stride_pack, int mid_dtype, int64_t M, int64_t N, int64_t K,
+                                     void* stream);
+
+/*
  * Upper bound on the SMs the persistent kernels of this library occupy (their grids are sized by the SM count), for
  * the calling process; 0 = all.  Returns the previous value.  A row-parallel linear that overlaps the all-reduce of
  * one row chunk with the GEMM of the next leaves a few SMs to the all-reduce kernel this way (the reference reaches

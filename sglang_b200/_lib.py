@@ -107,6 +107,17 @@ _SIGNATURES = {
     "b200_ep_combine": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                 c_int64, c_void_p, c_void_p, c_void_p]),
     "b200_debug_force_block_n": (c_int, [c_int]),
+    "b200_sm_count": (c_int, []),
+    "b200_fp8_linear_workspace_bytes": (ctypes.c_size_t, [c_int64, c_int64, c_int64, c_int]),
+    "b200_fp8_linear": (c_int, [c_void_p, c_int, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int64,
+                                c_int64, c_int64, c_int64, c_int, c_void_p, ctypes.c_size_t, c_void_p]),
+    "b200_fused_experts_fp8_workspace_bytes": (ctypes.c_size_t, [c_int64, c_int64, c_int64, c_int, c_int, c_int]),
+    "b200_fused_experts_fp8": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
+                                       c_int64, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+                                       c_void_p, ctypes.c_size_t, c_void_p]),
+    "b200_fp8_gate_up_silu_quant_pow2": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p,
+                                                 c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_int64,
+                                                 c_int64, c_int64, c_void_p]),
 }
 
 
@@ -124,6 +135,21 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (sglang_b200/_host.so, built together with the CUDA library)."""
+    global _host
+    if _host is None:
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise ImportError(f"sglang_b200/_host.so does not load: build it with `python -m sglang_b200.build` ({e})") from e
+        _host = module
+    return _host
 
 
 def check(fn_name: str, code: int) -> None:

@@ -2,7 +2,8 @@
 
     python -m sglang_b200.build [--force] [--verbose]
 
-The library has no torch dependency; it links only the CUDA runtime.  Object files go to
+The library has no torch dependency; it links only the CUDA runtime.  The host module (_host.so) is the torch-facing
+side: allocation and one C call per public function.  Object files go to
 sglang_b200/csrc/_build/, the shared library next to this file.
 """
 from __future__ import annotations
@@ -18,6 +19,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(CSRC, "_build")
 LIB = os.path.join(PKG, "libb200_block_fp8.so")
+HOST = os.path.join(PKG, "_host.so")
 HEADER = os.path.join(os.path.dirname(PKG), "include", "b200_block_fp8.h")
 
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
@@ -27,6 +29,30 @@ NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-gencode", "arch=compute_100a,c
 def _nvcc() -> str:
     cand = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "bin", "nvcc")
     return cand if os.path.isfile(cand) else "nvcc"
+
+
+def build_host(force: bool = False) -> str:
+    """The native host path: a CPython module against the installed torch's headers, linked to the CUDA library."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+    src = os.path.join(CSRC, "torch_host.cpp")
+    if not force and os.path.isfile(HOST) and os.path.getmtime(HOST) >= max(map(os.path.getmtime, (src, HEADER, __file__))):
+        return HOST
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) or "/usr/local/cuda"
+    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", src, "-o", HOST,
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for d in include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]:
+        cmd += ["-isystem", d]
+    for d in library_paths() + [PKG]:
+        cmd += ["-L" + d]
+    cmd += ["-l:" + os.path.basename(LIB), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
+            "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"host module build failed:\n{r.stderr}")
+    return HOST
 
 
 def sources():
@@ -97,6 +123,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stderr}")
+    build_host(force)
     return LIB
 
 

@@ -55,6 +55,8 @@ extern "C" int b200_set_sm_limit(int sms) {
   return old;
 }
 
+extern "C" int b200_sm_count(void) { return b200::sm_count(); }
+
 extern "C" const char* b200_strerror(int code) {
   switch (code) {
     case B200_OK: return "ok";

@@ -177,8 +177,8 @@ __device__ __forceinline__ MxTile mx_get_tile(int tile, const MxParams& p, int m
       sub = local / n_blocks;
       t.n_blk = local - sub * n_blocks;
     }
-    const int rows = __ldg(p.rows + static_cast<int64_t>(lo) * p.rows_stride);
-    const int off = __ldg(p.offsets + lo);
+    const int rows = p.rows ? __ldg(p.rows + static_cast<int64_t>(lo) * p.rows_stride) : p.M;   // no table: one problem
+    const int off = p.rows ? __ldg(p.offsets + lo) : 0;
     t.row0 = min(max(off + sub * TILE_M, 0), p.M - 1);
     t.sa_base = p.sa_stride_problem < 0 ? 0 : lo * p.sa_stride_problem - off * p.sa_stride_m;
     t.valid = max(1, min(min(TILE_M, rows - sub * TILE_M), p.M - t.row0));
@@ -227,7 +227,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if constexpr (GROUPED) {
     // row tiles per problem (none for an empty problem or one whose weight slice does not exist) ...
     for (int i = threadIdx.x; i < p.num_problems; i += blockDim.x) {
-      const int rows = __ldg(p.rows + static_cast<int64_t>(i) * p.rows_stride);
+      const int rows = p.rows ? __ldg(p.rows + static_cast<int64_t>(i) * p.rows_stride) : p.M;
       const int e = p.experts ? __ldg(p.experts + i) : i;
       tile_start[i + 1] = (rows > 0 && e >= 0 && e < p.num_weight_experts) ? (min(rows, p.M) + kTileM - 1) / kTileM : 0;
     }
@@ -1209,6 +1209,44 @@ extern "C" int b200_fp8_blockwise_scaled_grouped_mm_pow2_silu_quant(
   p.offsets = problem_offsets; p.rows = problem_rows; p.experts = problem_experts;
   p.rows_stride = problem_rows_stride; p.sb_stride_e = sb_stride_e; p.sa_stride_problem = sa_stride_problem;
   p.num_problems = num_problems; p.num_weight_experts = num_weight_experts;
+  p.out_s = out_s; p.out_s_stride_pack = out_s_stride_pack;
+  p.status = gemm_status_ptr();
+  if (!p.status) return B200_ERR_CUDA;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return mid_dtype == B200_DT_BF16 ? launch_mx_silu<__nv_bfloat16>(a, lda, b, ldb, p, st)
+                                    : launch_mx_silu<__half>(a, lda, b, ldb, p, st);
+}
+
+// The dense form of the above: one problem of M rows whose offset and count are in the parameter block instead of in
+// device memory (filling a one-entry table cost two kernels per call).
+extern "C" int b200_fp8_gate_up_silu_quant_pow2(const void* a, int64_t lda, const void* b, int64_t ldb,
+                                                const uint32_t* sa_packed, int64_t sa_stride_m, int64_t sa_stride_pack,
+                                                const float* sb_pow2, int64_t sb_stride_n, int64_t sb_stride_g, void* out_q,
+                                                int64_t ldq, uint32_t* out_s, int64_t out_s_stride_pack, int mid_dtype,
+                                                int64_t M, int64_t N, int64_t K, void* stream) {
+  using namespace b200;
+  if (M < 0 || N < 0 || K <= 0) return B200_ERR_BAD_SHAPE;
+  if (M == 0 || N == 0) return B200_OK;
+  if (M > 0x7fffff00LL || K > 0x7fffff00LL || 2 * N > 0x7fffff00LL) return B200_ERR_TOO_LARGE;
+  if (!a || !b || !sa_packed || !sb_pow2 || !out_q || !out_s) return B200_ERR_NULL_PTR;
+  if (mid_dtype != B200_DT_BF16 && mid_dtype != B200_DT_F16) return B200_ERR_BAD_DTYPE;
+  if (lda < K || ldb < K || ldq < N || out_s_stride_pack < M) return B200_ERR_BAD_STRIDE;
+  if ((lda % 16) != 0 || (ldb % 16) != 0 || (ldq % 16) != 0 || !aligned16(a) || !aligned16(b) || !aligned16(out_q))
+    return B200_ERR_MISALIGNED;
+  if (sa_stride_m < 0 || sa_stride_pack < 0 || sb_stride_n < 0 || sb_stride_g < 0) return B200_ERR_BAD_STRIDE;
+  if (K % 128 != 0) return B200_ERR_BAD_SHAPE;
+  if (N % 128 != 0) return B200_ERR_UNSUPPORTED;
+  int rc = require_sm100();
+  if (rc != B200_OK) return rc;
+  if (gemm_sticky_status() != 0) return B200_ERR_DEVICE_TIMEOUT;
+  MxParams p;
+  p.sa = sa_packed; p.sb = sb_pow2; p.out = out_q;
+  p.sa_stride_m = sa_stride_m; p.sa_stride_pack = sa_stride_pack;
+  p.sb_stride_n = sb_stride_n; p.sb_stride_g = sb_stride_g; p.ldo = ldq;
+  p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K);
+  p.out_dtype = mid_dtype;
+  p.offsets = nullptr; p.rows = nullptr; p.experts = nullptr;     // one problem: all M rows
+  p.rows_stride = 0; p.sb_stride_e = 0; p.sa_stride_problem = -1; p.num_problems = 1; p.num_weight_experts = 1;
   p.out_s = out_s; p.out_s_stride_pack = out_s_stride_pack;
   p.status = gemm_status_ptr();
   if (!p.status) return B200_ERR_CUDA;

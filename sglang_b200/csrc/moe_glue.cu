@@ -14,6 +14,8 @@
 // (a stable counting sort), one of the orders the reference can produce, and reproducible.
 // It runs as three launches over chunks of the flat id list and needs a scratch table of
 // per-chunk, per-expert counts in global memory.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -217,10 +219,11 @@ silu_and_mul_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t rows, 
 }
 
 // ---- out[i] = sum_j factors[i*topk+j] * in[perm[i*topk+j]], j ascending, fp32 accumulate
-template <typename T>
+// (factors in T, or in fp32: rounded to T before use)
+template <typename T, typename F>
 __global__ void __launch_bounds__(256)
 unpermute_sum_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __restrict__ perm,
-                     const T* __restrict__ factors, int m, int topk, int row_len) {
+                     const F* __restrict__ factors, int m, int topk, int row_len) {
   const int i = blockIdx.x;
   if (i >= m) return;
   const int vec_per_row = row_len / 8;
@@ -231,7 +234,7 @@ unpermute_sum_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_
     for (int j = 0; j < topk; ++j) {
       const int src = perm[i * topk + j];
       if (src < 0) continue;   // masked expert (expert parallel): contributes nothing
-      const float w = factors ? Pack8<T>::to_float(factors[i * topk + j]) : 1.0f;
+      const float w = factors ? Pack8<T>::to_float(static_cast<T>(factors[i * topk + j])) : 1.0f;
       float f[8];
       Pack8<T>::unpack(__ldg(reinterpret_cast<const uint4*>(in + static_cast<int64_t>(src) * row_len) + v), f);
 #pragma unroll
@@ -441,32 +444,44 @@ extern "C" int b200_silu_and_mul(const void* x, void* out, int64_t rows, int64_t
   return B200_OK;
 }
 
-extern "C" int b200_apply_shuffle_mul_sum(const void* input, void* output, const int32_t* permutation,
-                                          const void* factors, int64_t m, int64_t topk, int64_t row_len, int dtype,
-                                          void* stream) {
-  using namespace b200;
+namespace b200 {
+namespace {
+template <typename F>
+int unpermute_sum(const void* input, void* output, const int32_t* permutation, const void* factors, int64_t m,
+                  int64_t topk, int64_t row_len, int dtype, cudaStream_t st) {
   if (m < 0 || topk <= 0 || row_len < 0) return B200_ERR_BAD_SHAPE;
   if (m == 0 || row_len == 0) return B200_OK;
   if (!input || !output || !permutation) return B200_ERR_NULL_PTR;
   if ((row_len % 8) != 0 || !aligned16(input) || !aligned16(output)) return B200_ERR_MISALIGNED;
   if (m > 0x7fffffffLL) return B200_ERR_TOO_LARGE;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   int threads = static_cast<int>(row_len / 8);
   threads = threads > 256 ? 256 : (threads < 32 ? 32 : (threads + 31) / 32 * 32);
-  if (dtype == B200_DT_BF16) {
-    unpermute_sum_kernel<__nv_bfloat16><<<static_cast<unsigned>(m), threads, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(input), static_cast<__nv_bfloat16*>(output), permutation,
-        static_cast<const __nv_bfloat16*>(factors), static_cast<int>(m), static_cast<int>(topk),
-        static_cast<int>(row_len));
-  } else if (dtype == B200_DT_F16) {
-    unpermute_sum_kernel<__half><<<static_cast<unsigned>(m), threads, 0, st>>>(
-        static_cast<const __half*>(input), static_cast<__half*>(output), permutation,
-        static_cast<const __half*>(factors), static_cast<int>(m), static_cast<int>(topk), static_cast<int>(row_len));
-  } else {
-    return B200_ERR_BAD_DTYPE;
-  }
+  auto go = [&](auto* in) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(in)>>;
+    using Factor = std::conditional_t<std::is_void_v<F>, T, F>;
+    unpermute_sum_kernel<T, Factor><<<static_cast<unsigned>(m), threads, 0, st>>>(
+        in, static_cast<T*>(output), permutation, static_cast<const Factor*>(factors), static_cast<int>(m),
+        static_cast<int>(topk), static_cast<int>(row_len));
+  };
+  if (dtype == B200_DT_BF16) go(static_cast<const __nv_bfloat16*>(input));
+  else if (dtype == B200_DT_F16) go(static_cast<const __half*>(input));
+  else return B200_ERR_BAD_DTYPE;
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
+}
+}  // namespace
+
+int unpermute_sum_f32_factors(const void* input, void* output, const int32_t* permutation, const float* factors, int64_t m,
+                              int64_t topk, int64_t row_len, int dtype, cudaStream_t stream) {
+  return unpermute_sum<float>(input, output, permutation, factors, m, topk, row_len, dtype, stream);
+}
+}  // namespace b200
+
+extern "C" int b200_apply_shuffle_mul_sum(const void* input, void* output, const int32_t* permutation,
+                                          const void* factors, int64_t m, int64_t topk, int64_t row_len, int dtype,
+                                          void* stream) {
+  return b200::unpermute_sum<void>(input, output, permutation, factors, m, topk, row_len, dtype,
+                                   static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------------------------------------

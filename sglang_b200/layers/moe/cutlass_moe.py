@@ -11,6 +11,7 @@ from typing import Optional
 
 import torch
 
+from ... import _lib
 from ...sgl_kernel import (apply_shuffle_mul_sum, fp8_blockwise_scaled_grouped_mm, prepare_moe_input,
                            shuffle_packed_scales, shuffle_rows, silu_and_mul)
 from ..quantization.deep_gemm_wrapper import grouped_gemm_pow2, grouped_gemm_pow2_silu_quant
@@ -102,6 +103,9 @@ def fused_experts_block_fp8(a, w13, w2, w13_scale, w2_scale, topk_weights, topk_
     """Convenience form with natural weight layouts: w13 [E, 2n, k], w2 [E, k, n] e4m3 contiguous,
     scales [E, 2n/128, k/128] and [E, k/128, n/128] -- what Fp8MoEMethod holds
     (python/sglang/srt/layers/quantization/fp8.py:1030-1065 passes the transposed views)."""
+    done = _lib.host().experts(a, w13, w2, w13_scale, w2_scale, topk_weights, topk_ids, None, None, None, False)
+    if done is not None:
+        return done
     return cutlass_fused_experts_fp8(a, w13.transpose(1, 2), w2.transpose(1, 2), w13_scale.transpose(1, 2),
                                      w2_scale.transpose(1, 2), topk_weights, topk_ids)
 
@@ -115,6 +119,10 @@ def fused_experts_block_fp8_ue8m0(a, w13, w2, w13_scale, w2_scale, topk_weights,
     SiLU*mul -> quant -> grouped GEMM -> weighted gather); here every expert's rows are packed without padding and
     the schedule reads offsets and counts on the device.  fuse_activation: SiLU*mul and the second quantisation run in
     the first GEMM's epilogue (same bits as the separate kernels)."""
+    if fuse_activation:
+        done = _lib.host().experts(a, w13, w2, w13_scale, w2_scale, topk_weights, topk_ids, None, None, None, True)
+        if done is not None:
+            return done
     assert topk_weights.shape == topk_ids.shape
     assert a.dtype in (torch.half, torch.bfloat16) and a.dim() == 2 and a.is_contiguous()
     E, n2, k = w13.shape

@@ -110,6 +110,9 @@ def gate_up_silu_quant_pow2(a: torch.Tensor, sa_packed: torch.Tensor, w_gate_up:
     python/sglang/srt/layers/linear.py:415-520), ws [2n/128, K/128] fp32 powers of two.  One kernel computes the
     projection, SiLU(gate) * up and the quantisation for the down projection; returns (codes [M, n], packed exponents).
     Same bits as the GEMM into a `mid_dtype` tensor followed by silu_and_mul_per_token_group_quant_fp8."""
+    done = _lib.host().gate_up_silu_quant(a, sa_packed, w_gate_up, ws, mid_dtype)
+    if done is not None:
+        return done
     M = a.shape[0]
     dev = a.device
     offsets = torch.zeros(1, dtype=torch.int32, device=dev)

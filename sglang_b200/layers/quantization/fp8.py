@@ -21,6 +21,7 @@ from typing import Any, Dict, List, Optional
 
 import torch
 
+from ... import _lib
 from .fp8_utils import (deepgemm_w8a8_block_fp8_linear_with_fallback, dispatch_w8a8_block_fp8_linear,
                         requant_weight_ue8m0_inplace)
 
@@ -149,7 +150,7 @@ class Fp8LinearMethod:
             layer.weight_scale_is_ue8m0 = True
 
     def apply(self, layer: torch.nn.Module, x: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-        if getattr(layer, "weight_scale_is_ue8m0", False):
+        if layer.__dict__.get("weight_scale_is_ue8m0", False):
             return deepgemm_w8a8_block_fp8_linear_with_fallback(
                 input=x, weight=layer.weight, block_size=self.quant_config.weight_block_size,
                 weight_scale=layer.weight_scale_inv, input_scale=None, bias=bias, scale_ue8m0=True,
@@ -205,6 +206,13 @@ class Fp8MoEMethod:
         from ..moe.cutlass_moe import cutlass_fused_experts_fp8
         assert activation == "silu", "only SiLU gating is built"
         topk_weights, topk_ids = topk_output[0], topk_output[1]
+        output = _lib.host().experts(x, layer.w13_weight, layer.w2_weight, layer.w13_weight_scale_inv,
+                                     layer.w2_weight_scale_inv, topk_weights, topk_ids, self.expert_offsets,
+                                     self.problem_sizes1, self.problem_sizes2, False)
+        if output is not None:
+            if routed_scaling_factor is not None:
+                output *= routed_scaling_factor
+            return output
         output = cutlass_fused_experts_fp8(
             x, layer.w13_weight.transpose(1, 2), layer.w2_weight.transpose(1, 2),
             layer.w13_weight_scale_inv.transpose(1, 2), layer.w2_weight_scale_inv.transpose(1, 2),

@@ -13,6 +13,7 @@ from typing import List, Optional, Tuple
 import torch
 
 from ...sgl_kernel import fp8_blockwise_scaled_mm, sgl_per_token_group_quant_fp8
+from ...sgl_kernel import gemm
 from ...sgl_kernel.gemm import launch_dense_mm
 from ... import _lib
 
@@ -45,6 +46,9 @@ def create_per_token_group_quant_fp8_output_scale(x_shape, device, group_size, c
 def sglang_per_token_group_quant_fp8(x: torch.Tensor, group_size: int, eps: float = 1e-10,
                                      column_major_scales: bool = False, scale_tma_aligned: bool = False,
                                      scale_ue8m0: bool = False) -> Tuple[torch.Tensor, torch.Tensor]:
+    done = _lib.host().quant(x, group_size, eps, column_major_scales, scale_tma_aligned, scale_ue8m0)
+    if done is not None:
+        return done
     assert x.shape[-1] % group_size == 0, "the last dimension of `x` cannot be divisible by `group_size`"
     assert x.is_contiguous(), "`x` is not contiguous"
     x_q = torch.empty_like(x, device=x.device, dtype=fp8_dtype)
@@ -153,6 +157,10 @@ def rmsnorm_per_token_group_quant_fp8(x: torch.Tensor, weight: torch.Tensor, nor
     to rmsnorm(...) followed by sglang_per_token_group_quant_fp8(...), without writing and re-reading the normalised
     activations.  Returns (codes, scales) or (codes, scales, normed) with return_normed."""
     assert group_size == 128, "the fused form is built for 128-wide groups"
+    if not return_normed:
+        done = _lib.host().norm_quant(x, weight, norm_eps, residual, eps, column_major_scales, scale_tma_aligned, scale_ue8m0)
+        if done is not None:
+            return done
     _, y, q, s = _rmsnorm_launch(x, weight, norm_eps, residual, want_y=return_normed, want_q=True, eps=eps,
                                  column_major_scales=column_major_scales, scale_tma_aligned=scale_tma_aligned,
                                  scale_ue8m0=scale_ue8m0)
@@ -203,6 +211,10 @@ def w8a8_block_fp8_matmul(A: torch.Tensor, B: torch.Tensor, As: torch.Tensor, Bs
     assert len(block_size) == 2
     block_n, block_k = block_size
     assert block_n == 128 and block_k == 128, "only 128x128 weight blocks are built"
+    if gemm.SPLIT_K_MODE == "auto":
+        done = _lib.host().matmul(A, B, As, Bs, output_dtype)
+        if done is not None:
+            return done
     assert A.shape[-1] == B.shape[-1]
     assert A.shape[:-1] == As.shape[:-1]
     assert A.is_contiguous()
@@ -237,6 +249,9 @@ def w8a8_block_fp8_matmul_deepgemm(A: torch.Tensor, B: torch.Tensor, As: torch.T
     assert list(block_size) == [128, 128] and output_dtype == torch.bfloat16
     if As.dtype != torch.int32:
         return w8a8_block_fp8_matmul(A, B, As, Bs, block_size, output_dtype)
+    done = _lib.host().matmul_packed(A, B, As, Bs, weight_scale_ue8m0)
+    if done is not None:
+        return done
     assert A.dim() == 2 and A.is_contiguous() and B.dim() == 2 and B.is_contiguous()
     M, K = A.shape
     N = B.shape[0]

@@ -10,7 +10,8 @@ from typing import Callable, List, Optional
 
 import torch
 
-from ...sgl_kernel import fp8_blockwise_scaled_mm
+from ... import _lib
+from ...sgl_kernel import fp8_blockwise_scaled_mm, gemm
 from .fp8_kernel import sglang_per_token_group_quant_fp8, w8a8_block_fp8_matmul, w8a8_block_fp8_matmul_deepgemm
 
 
@@ -42,6 +43,10 @@ def w8a8_block_fp8_linear(input: torch.Tensor, weight: torch.Tensor, block_size:
     """`out` (extension): a row-major [tokens, N] tensor of the input dtype to write into."""
     assert input_scale is None
     assert list(block_size) == [128, 128]
+    if gemm.SPLIT_K_MODE == "auto":
+        done = _lib.host().linear(input, weight, weight_scale, bias, out, 0)
+        if done is not None:
+            return done
     if weight.shape[0] % 128 != 0 or weight.shape[1] % 128 != 0:
         y = ragged_w8a8_block_fp8_linear(input, weight, block_size, weight_scale, input_scale, bias)
         if out is not None:
@@ -108,6 +113,10 @@ def deepgemm_w8a8_block_fp8_linear_with_fallback(input: torch.Tensor, weight: to
     power-of-two weight scales too (requant_weight_ue8m0): the product then runs on the tensor core's
     block-scaling path, all k-blocks accumulated in tensor memory."""
     assert input_scale is None
+    if scale_ue8m0 and list(block_size) == [128, 128]:
+        done = _lib.host().linear(input, weight, weight_scale, bias, None, 2 if weight_scale_ue8m0 else 1)
+        if done is not None:
+            return done
     if not (input.dtype == torch.bfloat16 and weight.shape[0] % 64 == 0 and weight.shape[1] % 128 == 0
             and weight.shape[0] % 128 == 0):
         return w8a8_block_fp8_linear(input, weight, block_size, weight_scale, input_scale, bias)

@@ -85,6 +85,10 @@ def moe_fused_gate(input_tensor: torch.Tensor, bias: torch.Tensor, num_expert_gr
     topk slots are the fused shared experts: ids num_experts, num_experts + 1, ..., weight
     1 / routed_scaling_factor; the routed slots before them are renormalised over themselves
     (sgl-kernel/csrc/moe/moe_fused_gate.cu:225-252)."""
+    done = _lib.host().fused_gate(input_tensor, bias, num_expert_group, topk_group, topk, num_fused_shared_experts,
+                                  routed_scaling_factor)
+    if done is not None:
+        return done
     _check(0 <= num_fused_shared_experts < topk, "num_fused_shared_experts must be smaller than topk")
     _check(num_fused_shared_experts == 0 or routed_scaling_factor != 0, "routed_scaling_factor must be non-zero")
     _check(input_tensor.is_cuda and bias.is_cuda, "tensors must be CUDA tensors")
@@ -204,6 +208,10 @@ def apply_shuffle_mul_sum(input, output, permutation, factors):
 def silu_and_mul(input: torch.Tensor, out: torch.Tensor = None) -> torch.Tensor:
     if input.shape[-1] * input.dtype.itemsize % 16 != 0:
         raise ValueError("The pointers must be multiple of 16 bytes.")
+    if out is None:
+        done = _lib.host().silu_and_mul(input)
+        if done is not None:
+            return done
     d = input.shape[-1] // 2
     if out is None:
         out = torch.empty(input.shape[:-1] + (d,), device=input.device, dtype=input.dtype)
