@@ -448,6 +448,9 @@ int b200_fp8_linear(const void* x, int dtype, const void* w, int64_t ldw, const 
                     int64_t ws_stride_g, const void* bias, void* out, int64_t ldo, int64_t M, int64_t N, int64_t K,
                     int scale_mode, void* workspace, size_t workspace_bytes, void* stream);
 int b200_sm_count(void);
+/* Workspace with which b200_fp8_blockwise_scaled_mm_splitk (split_k = 0) runs its best schedule on the current device;
+ * with less it splits less. */
+size_t b200_fp8_blockwise_scaled_mm_workspace_bytes(int64_t M, int64_t N, int64_t K);
 
 /*
  * The fused expert layer, start to finish (cutlass_fused_experts_fp8, python/sglang/srt/layers/moe/cutlass_moe.py:29-222):

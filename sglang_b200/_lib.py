@@ -108,6 +108,7 @@ _SIGNATURES = {
                                 c_int64, c_void_p, c_void_p, c_void_p]),
     "b200_debug_force_block_n": (c_int, [c_int]),
     "b200_sm_count": (c_int, []),
+    "b200_fp8_blockwise_scaled_mm_workspace_bytes": (ctypes.c_size_t, [c_int64, c_int64, c_int64]),
     "b200_fp8_linear_workspace_bytes": (ctypes.c_size_t, [c_int64, c_int64, c_int64, c_int]),
     "b200_fp8_linear": (c_int, [c_void_p, c_int, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int64,
                                 c_int64, c_int64, c_int64, c_int, c_void_p, ctypes.c_size_t, c_void_p]),

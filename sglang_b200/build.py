@@ -68,7 +68,7 @@ def _deps_mtime() -> float:
 # assumes the launch allocates exactly this many registers per thread.  If ptxas ever allocates fewer,
 # setmaxnreg.inc would wait for registers nobody releases, so the build refuses the object instead.
 _FIXED_REGS = [
-    (re.compile(r"gemm_block_fp8_kernelILi(128|256)ELi16E"), 96),
+    (re.compile(r"gemm_block_fp8_kernelILb"), 168),
     (re.compile(r"gemm_block_fp8_swapab_kernelILi128E"), 168),
 ]
 

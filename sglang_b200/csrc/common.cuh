@@ -155,6 +155,70 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, i
   return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
 }
 
+// ---- the same operations on 32-bit shared-window addresses.  A pointer into dynamic shared memory that was aligned by
+// integer arithmetic is a GENERIC pointer to the compiler: loads through it take the slow path and every barrier operation
+// converts a 64-bit address.  Kernels whose inner loops synchronise per k-block keep 32-bit addresses instead.
+namespace sa {
+__device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Bounded by a count of tries (a failed try suspends the thread in hardware for a while, so the limit is seconds): no
+// clock reads and one register in the loop.
+constexpr uint32_t kWaitTries = 1u << 26;
+__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, int* status, int code) {
+  for (uint32_t n = 0; n < kWaitTries; ++n)
+    if (try_wait(bar, parity)) return true;
+  report_wait_failure(status, code);
+  return false;
+}
+__device__ __forceinline__ void arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void arrive_if(uint32_t bar, bool p) {   // predicated, no branch
+  asm volatile("{\n\t.reg .pred P;\n\tsetp.ne.b32 P, %1, 0;\n\t@P mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}\n"
+               ::"r"(bar), "r"(p ? 1 : 0) : "memory");
+}
+__device__ __forceinline__ void expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ float ld_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+// Asynchronous 4- and 16-byte copies global -> shared (zero-filled when !in), and the arrival on `bar` once all of this
+// thread's earlier ones have landed (counted in the barrier's init count).
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+}  // namespace sa
+
 // ---- TMA (tiled bulk tensor copy global -> shared, completion on an mbarrier; no multicast)
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(

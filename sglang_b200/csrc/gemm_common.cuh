@@ -24,10 +24,13 @@ struct GemmParams {
   int split_k;
   int kb_per_split;
   float* partial;
-  // tail split (dense, large M): tiles [0, tail_first) are whole; each tile from tail_first on -- the ones
-  // that would form a mostly empty last wave -- is divided among split_k CTAs, partial sums stored compactly
-  // as partial[(tile - tail_first) * split_k + split][128][block_n].  0 = the uniform split above.
+  // tail split (dense, CTA-pair kernel): tiles [0, tail_first) are whole; each tile from tail_first on -- the ones
+  // that would form a mostly empty last wave -- is divided among split_k pairs.  partial_tiles != 0: partial sums are
+  // whole tiles, partial[(tile - tail_first) * split_k + split][256][tile_n]
   int tail_first;
+  int partial_tiles;
+  const void* bias; // [N] in the output type, added to the rounded product; or nullptr
+  int tile_n;       // tile width of the CTA-pair kernel, 128 or 256
   // activation scales given as packed UE8M0 exponent bytes (four k-blocks per 32-bit word) instead of fp32:
   // element (m, kb) is byte kb % 4 of the word at sa[(kb / 4) * sa_stride_g + m * sa_stride_m]
   int sa_ue8m0;
@@ -69,6 +72,13 @@ __device__ __forceinline__ __nv_bfloat16 cvt1(__nv_bfloat16*, float a) { return 
 __device__ __forceinline__ __half cvt1(__half*, float a) { return __float2half_rn(a); }
 __device__ __forceinline__ float cvt1(float*, float a) { return a; }
 
+// 32 bytes to a 32-byte-aligned address in one store: a warp that writes one row per lane then fills whole sectors.
+__device__ __forceinline__ void st_global_32(void* dst, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+
 // Store NCOLS consecutive outputs of one row; `valid` = columns left before N.
 template <int NCOLS, typename OutT>
 __device__ __forceinline__ void store_row(OutT* dst, const float (&acc)[NCOLS], int valid, bool vec_ok) {
@@ -98,6 +108,35 @@ __device__ __forceinline__ void store_row(float* dst, const float (&acc)[NCOLS],
 #pragma unroll
     for (int c = 0; c < NCOLS; ++c)
       if (c < valid) dst[c] = acc[c];
+  }
+}
+
+// One thread's row segment of the output, `cols` of NCOLS columns from (m, n0) on, 16 columns at a time: 32-byte stores
+// where the row allows them (full sectors: 60 cycles per k-block of a 128 x 256 tile less than 16-byte ones).  The bias
+// is added to the value rounded to the output type, as `out += bias` does.
+template <int NCOLS, typename OutT>
+__device__ __forceinline__ void store_out(OutT* out, const OutT* bias, int64_t m, int n0, int64_t ldo, float (&acc)[NCOLS], int cols) {
+  OutT* dst = out + m * ldo + n0;
+  if (bias != nullptr) {
+#pragma unroll
+    for (int c = 0; c < NCOLS; ++c)
+      if (c < cols) acc[c] = static_cast<float>(cvt1(dst, acc[c])) + static_cast<float>(bias[n0 + c]);
+  }
+  const bool vec16 = ((ldo * sizeof(OutT)) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  const bool vec32 = ((ldo * sizeof(OutT)) & 31) == 0 && (reinterpret_cast<uintptr_t>(out) & 31u) == 0;
+#pragma unroll
+  for (int c = 0; c < NCOLS; c += 16) {
+    if (c >= cols) break;
+    if constexpr (sizeof(OutT) == 2) {
+      if (vec32 && cols - c >= 16) {
+        uint32_t v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = pack2(dst, acc[c + 2 * i], acc[c + 2 * i + 1]);
+        st_global_32(dst + c, v);
+        continue;
+      }
+    }
+    store_row<16>(dst + c, reinterpret_cast<const float(&)[16]>(acc[c]), cols - c, vec16);
   }
 }
 

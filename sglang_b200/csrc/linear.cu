@@ -78,10 +78,7 @@ LinearPlan plan_linear(Arena& a, int64_t M, int64_t N, int64_t K, bool ue8m0) {
   p.q = a.take<uint8_t>(static_cast<size_t>(M) * K);
   p.s_ld = align4(M);
   p.s = a.take<uint32_t>(static_cast<size_t>(p.s_ld) * (ue8m0 ? (groups + 3) / 4 : groups));
-  int split = 1;
-  size_t bytes = 0;
-  if (!ue8m0) b200_fp8_blockwise_scaled_mm_splitk_plan(M, N, K, sm_count(), &split, &bytes);
-  p.partial_bytes = split > 1 ? bytes : 0;
+  p.partial_bytes = ue8m0 ? 0 : b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K);
   p.partial = p.partial_bytes ? a.take<uint8_t>(p.partial_bytes) : nullptr;
   return p;
 }

@@ -259,15 +259,13 @@ HOST_FN(matmul) {
   if (w->device() != dev || xs->device() != dev || ws->device() != dev) return none();
   const c10::cuda::OptionalCUDAGuard guard(dev);
   Tensor out = empty({M, N}, ot, dev);
-  int split = 1;
-  size_t bytes = 0;
-  b200_fp8_blockwise_scaled_mm_splitk_plan(M, N, K, b200_sm_count(), &split, &bytes);
+  const size_t bytes = b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K);
   Tensor work;
-  if (split > 1) work = empty({static_cast<int64_t>(bytes)}, at::kByte, dev);
+  if (bytes) work = empty({static_cast<int64_t>(bytes)}, at::kByte, dev);
   const int rc = b200_fp8_blockwise_scaled_mm_splitk(
       x->data_ptr(), K, w->data_ptr(), K, static_cast<const float*>(xs->data_ptr()), xs->stride(0), xs->stride(1),
       static_cast<const float*>(ws->data_ptr()), ws->stride(0), ws->stride(1), out.data_ptr(), N, dt_of(ot), M, N, K, 0,
-      split > 1 ? work.data_ptr() : nullptr, split > 1 ? bytes : 0, stream_of(dev));
+      bytes ? work.data_ptr() : nullptr, bytes, stream_of(dev));
   if (rc != 0) return raise_status("w8a8_block_fp8_matmul", rc);
   return THPVariable_Wrap(std::move(out));
 }

@@ -34,7 +34,6 @@ def _is_contiguous_vector(t: torch.Tensor) -> bool:
     return t.is_contiguous() and (t.dim() == 1 or (t.dim() == 2 and min(t.shape) == 1))
 
 
-_SM_COUNT: dict = {}
 _WORKSPACE: dict = {}
 # Split-K for decode-size batches: "auto" lets the library choose, "off" always runs the unsplit kernel.
 SPLIT_K_MODE = "auto"
@@ -54,7 +53,7 @@ def set_sm_limit(sms: int) -> int:
 
 
 def _splitk_plan(M: int, N: int, K: int, device: torch.device):
-    """Split count and workspace bytes the library chooses for this shape (1, 0 = no split): all tiles
+    """(whether the library would split k-blocks for this shape: > 1, workspace bytes it wants for that): all tiles
     for decode-size M on narrow deep projections, only the last wave of tiles for large M when that wave
     would be mostly empty.  Cached per shape and device."""
     if SPLIT_K_MODE != "auto":
@@ -64,16 +63,8 @@ def _splitk_plan(M: int, N: int, K: int, device: torch.device):
     hit = _PLAN.get(key)
     if hit is not None:
         return hit
-    sms = _SM_COUNT.get(idx)
-    if sms is None:
-        sms = _SM_COUNT[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
-    if _SM_LIMIT > 0:
-        sms = min(sms, _SM_LIMIT)
-    import ctypes
-    s, b = ctypes.c_int(1), ctypes.c_size_t(0)
-    _lib.check("fp8_blockwise_scaled_mm_splitk_plan",
-               _lib.lib().b200_fp8_blockwise_scaled_mm_splitk_plan(M, N, K, sms, ctypes.byref(s), ctypes.byref(b)))
-    _PLAN[key] = (s.value, b.value)
+    nbytes = _lib.lib().b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K)
+    _PLAN[key] = (2 if nbytes else 1, nbytes)
     return _PLAN[key]
 
 
