@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "../../include/b200_block_fp8.h"
 
 namespace b200 {
@@ -34,11 +36,42 @@ int sm_count();
 // 0 if the current device is compute capability 10.x, else B200_ERR_NOT_SM100 / B200_ERR_CUDA.
 int require_sm100();
 
+#if defined(__CUDACC__)
+// Launch with programmatic stream serialisation: the kernel may become resident while the one before it in the stream
+// still runs.  Such a kernel calls pdl_wait() before it touches global memory (the wait ends when everything earlier in
+// the stream has completed and is visible), so results do not depend on the overlap; it hides the launch gap and the
+// kernel's own prologue, 1-3 us per kernel, which is most of a decode-size call.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+#endif
+
 // ----------------------------------------------------------------------------- device side
 #if defined(__CUDACC__)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// Programmatic dependent launch.  pdl_wait: everything earlier in the stream has completed and is visible.  pdl_trigger:
+// the next kernel's blocks may become resident; issued after the wait, so that what a dependent reads BEFORE its own wait
+// (weights, in a chain this library launches) was complete before this kernel began.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_start() {
+  pdl_wait();
+  pdl_trigger();
 }
 
 __device__ __forceinline__ bool elect_one() {

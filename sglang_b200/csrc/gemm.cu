@@ -140,29 +140,6 @@ __device__ __forceinline__ Work decode_work(int vt, const GemmParams& p, int nkb
   return Work{tile, split, kb0, min(nkb, kb0 + p.kb_per_split), true};
 }
 
-// Row-tile prefix table of the grouped form, by the whole CTA: per-expert counts, then a warp's running sum.
-__device__ __forceinline__ void build_tile_table(int* tile_start, const int32_t* problem_sizes, int num_experts, int tile_rows) {
-  for (int e = threadIdx.x; e < num_experts; e += blockDim.x)
-    tile_start[e + 1] = (max(problem_sizes[e * 3], 0) + tile_rows - 1) / tile_rows;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    int carry = 0;
-    for (int base = 0; base < num_experts; base += 32) {
-      int v = (base + lane < num_experts) ? tile_start[base + lane + 1] : 0;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, v, off);
-        if (lane >= off) v += u;
-      }
-      if (base + lane < num_experts) tile_start[base + lane + 1] = carry + v;
-      carry += __shfl_sync(0xffffffffu, v, 31);
-    }
-    if (lane == 0) tile_start[0] = 0;
-  }
-  __syncthreads();
-}
-
 template <bool GROUPED, typename OutT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -186,7 +163,10 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const int n_blocks = (p.N + p.tile_n - 1) / p.tile_n;
   const int nkb = (p.K + BLOCK_K - 1) / BLOCK_K;
 
-  if constexpr (GROUPED) build_tile_table(tile_m_start, p.problem_sizes, p.num_experts, TILE_M);
+  if constexpr (GROUPED) {
+    pdl_start();     // the tables come from the kernels before this one
+    build_tile_table(tile_m_start, p.problem_sizes, p.num_experts, TILE_M);
+  }
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
@@ -228,23 +208,46 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
+    int ahead = 0;     // k-blocks of the first unit whose weights are on their way already
+    if constexpr (!GROUPED) {
+      if (p.prefetch_w && blockIdx.x < num_vtiles) {
+        const Work w = decode_work(blockIdx.x, p, nkb, GROUPED);
+        const TileInfo t = get_tile<GROUPED>(w.tile, p, m_blocks, n_blocks, tile_m_start);
+        ahead = min(kStages, w.kb_end - w.kb_begin);
+        if (elect_one()) {
+          for (int i = 0; i < ahead; ++i) {
+            const uint32_t bar = full_bar + 8 * i;
+            sa::expect_tx(bar, kABytes + t.halves * kBHalfBytes);
+            for (int h = 0; h < t.halves; ++h)
+              sa::tma_load_2d(smem_b + i * kBBytes + h * kBHalfBytes, &map_b, bar, (w.kb_begin + i) * BLOCK_K, t.b_row0 + h * 128);
+          }
+        }
+        __syncwarp();
+      }
+      pdl_start();
+    }
     for (int vt = blockIdx.x; ok && vt < num_vtiles; vt += gridDim.x) {
       const Work w = decode_work(vt, p, nkb, GROUPED);
       const TileInfo t = get_tile<GROUPED>(w.tile, p, m_blocks, n_blocks, tile_m_start);
       const uint32_t bytes = kABytes + t.halves * kBHalfBytes;
       for (int kb = w.kb_begin; kb < w.kb_end; ++kb) {
-        ok = sa::wait(done_bar + 8 * stage, phase ^ 1u, p.status, 1);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+        if (ahead == 0) {
+          ok = sa::wait(done_bar + 8 * stage, phase ^ 1u, p.status, 1);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+        }
         if (elect_one()) {
           const uint32_t bar = full_bar + 8 * stage;
-          sa::expect_tx(bar, bytes);
+          if (ahead == 0) {
+            sa::expect_tx(bar, bytes);
+            sa::tma_load_2d(smem_b + stage * kBBytes, &map_b, bar, kb * BLOCK_K, t.b_row0);
+            if (t.halves == 2)
+              sa::tma_load_2d(smem_b + stage * kBBytes + kBHalfBytes, &map_b, bar, kb * BLOCK_K, t.b_row0 + 128);
+          }
           sa::tma_load_2d(smem_a + stage * kABytes, &map_a, bar, kb * BLOCK_K, t.row0);
-          sa::tma_load_2d(smem_b + stage * kBBytes, &map_b, bar, kb * BLOCK_K, t.b_row0);
-          if (t.halves == 2)
-            sa::tma_load_2d(smem_b + stage * kBBytes + kBHalfBytes, &map_b, bar, kb * BLOCK_K, t.b_row0 + 128);
         }
         __syncwarp();
+        if (ahead > 0) --ahead;
         if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
     }
@@ -286,7 +289,8 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
     __syncwarp();
   } else if (warp == kStagerWarp) {
-    // ------------------------------------------------------------------ scale stager (each CTA, its own rows)
+    // ------------------------------------------------------------------ scale stager
+    if constexpr (!GROUPED) pdl_wait();
     int slot = 0;
     uint32_t sphase = 0;
     bool ok = true;
@@ -470,7 +474,9 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 // CTA finished first), converted to the output type.  One thread per four consecutive columns.
 template <typename OutT>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ partial, OutT* __restrict__ out,
-                                                            int M, int N, int64_t ldo, int split_k) {
+                                                            const OutT* __restrict__ bias, int M, int N, int64_t ldo,
+                                                            int split_k) {
+  pdl_start();
   const int n4 = N >> 2;
   const int64_t total = static_cast<int64_t>(M) * n4;
   const int64_t plane = static_cast<int64_t>(M) * N;
@@ -484,7 +490,13 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
     OutT* dst = out + static_cast<int64_t>(m) * ldo + c;
-    dst[0] = cvt1(dst, acc.x); dst[1] = cvt1(dst, acc.y); dst[2] = cvt1(dst, acc.z); dst[3] = cvt1(dst, acc.w);
+    const float vals[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      OutT v = cvt1(dst, vals[j]);
+      if (bias) v = cvt1(dst, static_cast<float>(v) + static_cast<float>(bias[c + j]));
+      dst[j] = v;
+    }
   }
 }
 
@@ -493,7 +505,8 @@ int launch_reduce(const GemmParams& p, cudaStream_t stream) {
   const int64_t total = static_cast<int64_t>(p.M) * (p.N >> 2);
   int64_t blocks = (total + 255) / 256;
   if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
-  splitk_reduce_kernel<OutT><<<static_cast<int>(blocks), 256, 0, stream>>>(p.partial, static_cast<OutT*>(p.out), p.M, p.N,
+  launch_pdl(splitk_reduce_kernel<OutT>, static_cast<int>(blocks), 256, 0, stream, p.partial, static_cast<OutT*>(p.out),
+             static_cast<const OutT*>(p.bias), p.M, p.N,
                                                                          p.ldo, p.split_k);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
@@ -505,8 +518,9 @@ int launch_reduce(const GemmParams& p, cudaStream_t stream) {
 constexpr int kTailSlices = 16;
 template <typename OutT>
 __global__ void __launch_bounds__(256) tail_reduce_kernel(const float* __restrict__ partial, OutT* __restrict__ out,
-                                                          int M, int N, int64_t ldo, int split_k, int tail_first,
+                                                          const OutT* __restrict__ bias, int M, int N, int64_t ldo, int split_k, int tail_first,
                                                           int m_blocks, int n_blocks, int tile_n) {
+  pdl_start();
   int m_blk, n_blk;
   tile_coords(tail_first + blockIdx.x, m_blocks, n_blocks, m_blk, n_blk);
   const int64_t plane = static_cast<int64_t>(TILE_M) * tile_n;
@@ -527,7 +541,11 @@ __global__ void __launch_bounds__(256) tail_reduce_kernel(const float* __restric
     const float vals[4] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      if (n + j < N) dst[j] = cvt1(dst, vals[j]);
+      if (n + j < N) {
+        OutT v = cvt1(dst, vals[j]);
+        if (bias) v = cvt1(dst, static_cast<float>(v) + static_cast<float>(bias[n + j]));
+        dst[j] = v;
+      }
   }
 }
 
@@ -536,7 +554,8 @@ int launch_tail_reduce(const GemmParams& p, cudaStream_t stream) {
   const int m_blocks = (p.M + TILE_M - 1) / TILE_M;
   const int n_blocks = (p.N + p.tile_n - 1) / p.tile_n;
   const dim3 grid(m_blocks * n_blocks - p.tail_first, kTailSlices);
-  tail_reduce_kernel<OutT><<<grid, 256, 0, stream>>>(p.partial, static_cast<OutT*>(p.out), p.M, p.N, p.ldo, p.split_k,
+  launch_pdl(tail_reduce_kernel<OutT>, grid, 256, 0, stream, p.partial, static_cast<OutT*>(p.out),
+             static_cast<const OutT*>(p.bias), p.M, p.N, p.ldo, p.split_k,
                                                      p.tail_first, m_blocks, n_blocks, p.tile_n);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
@@ -571,8 +590,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, cu
                                   : split_from + (dense_tiles - split_from) * p.split_k;
   if (tiles > 0x7fffffffLL) return B200_ERR_TOO_LARGE;   // the kernels count tiles in 32 bits
   const int grid = tiles < sm_count() ? static_cast<int>(tiles) : sm_count();
-  kern<<<grid, kThreads, kSmemBytes, stream>>>(ma, mb, p);
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(kThreads), kSmemBytes, stream, ma, mb, p));
   return B200_OK;
 }
 
@@ -714,10 +732,12 @@ TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, size_t max_bytes) 
   return best;
 }
 
+}  // namespace
+
 int dense_mm(const void* a, int64_t lda, const void* b, int64_t ldb, const float* sa, int64_t sa_stride_m,
              int64_t sa_stride_g, const float* sb, int64_t sb_stride_n, int64_t sb_stride_g, void* out, int64_t ldo,
              int out_dtype, int64_t M, int64_t N, int64_t K, int split_k, void* workspace, size_t workspace_bytes,
-             void* stream, int sa_ue8m0 = 0) {
+             void* stream, int sa_ue8m0, const void* bias, int prefetch_w) {
   if (M < 0 || N < 0 || K <= 0) return B200_ERR_BAD_SHAPE;
   if (M == 0 || N == 0) return B200_OK;
   if (M > 0x7fffff00LL || N > 0x7fffff00LL || K > 0x7fffff00LL) return B200_ERR_TOO_LARGE;
@@ -772,7 +792,8 @@ int dense_mm(const void* a, int64_t lda, const void* b, int64_t ldb, const float
   p.split_k = (nkb + p.kb_per_split - 1) / p.kb_per_split;
   p.tail_first = 0;
   p.partial_tiles = 0;
-  p.bias = nullptr;
+  p.bias = bias;
+  p.prefetch_w = prefetch_w;
   p.tile_n = plan.tile_n;
   if (plan.split_k > 1) {
     p.split_k = plan.split_k;
@@ -805,7 +826,6 @@ int dense_mm(const void* a, int64_t lda, const void* b, int64_t ldb, const float
   return reduce_partials(p, st);
 }
 
-}  // namespace
 }  // namespace b200
 
 extern "C" int b200_fp8_blockwise_scaled_mm(const void* a, int64_t lda, const void* b, int64_t ldb, const float* sa,
@@ -813,7 +833,7 @@ extern "C" int b200_fp8_blockwise_scaled_mm(const void* a, int64_t lda, const vo
                                             int64_t sb_stride_n, int64_t sb_stride_g, void* out, int64_t ldo,
                                             int out_dtype, int64_t M, int64_t N, int64_t K, void* stream) {
   return b200::dense_mm(a, lda, b, ldb, sa, sa_stride_m, sa_stride_g, sb, sb_stride_n, sb_stride_g, out, ldo, out_dtype,
-                        M, N, K, 1, nullptr, 0, stream);
+                        M, N, K, 1, nullptr, 0, stream, 0, nullptr, 0);
 }
 
 extern "C" int b200_fp8_blockwise_scaled_mm_splitk(const void* a, int64_t lda, const void* b, int64_t ldb,
@@ -822,7 +842,7 @@ extern "C" int b200_fp8_blockwise_scaled_mm_splitk(const void* a, int64_t lda, c
                                                    int64_t ldo, int out_dtype, int64_t M, int64_t N, int64_t K,
                                                    int split_k, void* workspace, size_t workspace_bytes, void* stream) {
   return b200::dense_mm(a, lda, b, ldb, sa, sa_stride_m, sa_stride_g, sb, sb_stride_n, sb_stride_g, out, ldo, out_dtype,
-                        M, N, K, split_k, workspace, workspace_bytes, stream);
+                        M, N, K, split_k, workspace, workspace_bytes, stream, 0, nullptr, 0);
 }
 
 extern "C" int b200_fp8_blockwise_scaled_mm_ue8m0(const void* a, int64_t lda, const void* b, int64_t ldb,
@@ -831,7 +851,7 @@ extern "C" int b200_fp8_blockwise_scaled_mm_ue8m0(const void* a, int64_t lda, co
                                                   int64_t ldo, int out_dtype, int64_t M, int64_t N, int64_t K,
                                                   void* stream) {
   return b200::dense_mm(a, lda, b, ldb, reinterpret_cast<const float*>(sa_packed), sa_stride_m, sa_stride_pack, sb,
-                        sb_stride_n, sb_stride_g, out, ldo, out_dtype, M, N, K, 1, nullptr, 0, stream, 1);
+                        sb_stride_n, sb_stride_g, out, ldo, out_dtype, M, N, K, 1, nullptr, 0, stream, 1, nullptr, 0);
 }
 
 extern "C" int b200_fp8_blockwise_scaled_mm_splitk_plan(int64_t M, int64_t N, int64_t K, int sm_count, int* split_k,
@@ -887,7 +907,7 @@ extern "C" int b200_fp8_blockwise_scaled_grouped_mm(const void* a, int64_t lda, 
   p.status = gemm_status_ptr();
   p.expert_offsets = expert_offsets; p.problem_sizes = problem_sizes; p.num_experts = num_experts;
   p.split_k = 1; p.kb_per_split = 0; p.partial = nullptr; p.tail_first = 0; p.sa_ue8m0 = 0;
-  p.partial_tiles = 0; p.tile_n = 256; p.bias = nullptr;
+  p.partial_tiles = 0; p.tile_n = 256; p.bias = nullptr; p.prefetch_w = 0;
   if (!p.status) return B200_ERR_CUDA;
 
   // An expert's weights are rows [e*N, (e+1)*N) of one [E*N, K] matrix.

@@ -30,6 +30,8 @@ struct GemmParams {
   int tail_first;
   int partial_tiles;
   const void* bias; // [N] in the output type, added to the rounded product; or nullptr
+  int prefetch_w;   // != 0: the kernel before this one in the stream is this library's own and triggered after its wait, so
+                    // weights may be fetched ahead of the wait
   int tile_n;       // tile width of the CTA-pair kernel, 128 or 256
   // activation scales given as packed UE8M0 exponent bytes (four k-blocks per 32-bit word) instead of fp32:
   // element (m, kb) is byte kb % 4 of the word at sa[(kb / 4) * sa_stride_g + m * sa_stride_m]
@@ -45,7 +47,37 @@ int gemm_sticky_status();
 // box_rows x 128 bytes, 128-byte swizzle, zero fill outside the matrix.
 int make_map_u8_2d(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows);
 
+// The dense fp32-promotion GEMM behind the C entry points (gemm.cu).  split_k 0: the library's own schedule, as far as the
+// workspace allows; sa_ue8m0: packed exponent activation scales; bias and prefetch_w as in GemmParams.
+int dense_mm(const void* a, int64_t lda, const void* b, int64_t ldb, const float* sa, int64_t sa_stride_m,
+             int64_t sa_stride_g, const float* sb, int64_t sb_stride_n, int64_t sb_stride_g, void* out, int64_t ldo,
+             int out_dtype, int64_t M, int64_t N, int64_t K, int split_k, void* workspace, size_t workspace_bytes,
+             void* stream, int sa_ue8m0, const void* bias, int prefetch_w);
+
 #if defined(__CUDACC__)
+// Row-tile prefix table of the grouped form, by the whole CTA: per-expert counts, then a warp's running sum.
+__device__ __forceinline__ void build_tile_table(int* tile_start, const int32_t* problem_sizes, int num_experts, int tile_rows) {
+  for (int e = threadIdx.x; e < num_experts; e += blockDim.x)
+    tile_start[e + 1] = (max(problem_sizes[e * 3], 0) + tile_rows - 1) / tile_rows;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int carry = 0;
+    for (int base = 0; base < num_experts; base += 32) {
+      int v = (base + lane < num_experts) ? tile_start[base + lane + 1] : 0;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, off);
+        if (lane >= off) v += u;
+      }
+      if (base + lane < num_experts) tile_start[base + lane + 1] = carry + v;
+      carry += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) tile_start[0] = 0;
+  }
+  __syncthreads();
+}
+
 // Activation scale of (row, k-block), fp32 or packed UE8M0.  The representation is a template argument so
 // that a stager's batch of loads stays a straight line of independent loads: with a run-time test inside
 // every load the compiler serialised them and the stager fell behind the tensor pipe.

@@ -151,17 +151,8 @@ gemm_block_fp8_swapab_kernel(const __grid_constant__ CUtensorMap map_w, const __
   const int nkb = (p.K + BLOCK_K - 1) / BLOCK_K;
 
   if constexpr (GROUPED) {
-    for (int e = threadIdx.x; e < p.num_experts; e += blockDim.x)
-      tile_start[e + 1] = (max(p.problem_sizes[e * 3], 0) + TN - 1) / TN;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int run = 0;
-      tile_start[0] = 0;
-      for (int e = 1; e <= p.num_experts; ++e) {
-        run += tile_start[e];
-        tile_start[e] = run;
-      }
-    }
+    pdl_start();     // the tables come from the kernels before this one
+    build_tile_table(tile_start, p.problem_sizes, p.num_experts, TN);
   }
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::kStages; ++i) {
@@ -201,23 +192,43 @@ gemm_block_fp8_swapab_kernel(const __grid_constant__ CUtensorMap map_w, const __
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
+    int ahead = 0;     // stages of the first unit whose weights are on their way already
+    if constexpr (!GROUPED) {
+      if (p.prefetch_w && blockIdx.x < num_vtiles) {
+        const SwapTile t = get_swap_tile<GROUPED, TN>(blockIdx.x / split_k, p, m_tiles, n_tiles, tile_start);
+        const int kb_begin = (blockIdx.x % split_k) * kbps, kb_end = min(nkb, kb_begin + kbps);
+        ahead = min(C::kStages, (kb_end - kb_begin + kPair - 1) / kPair);
+        if (elect_one()) {
+          for (int i = 0; i < ahead; ++i) {
+            const int kb = kb_begin + i * kPair, n = min(kPair, kb_end - kb);
+            mbar_expect_tx(&full_bar[i], n * (C::kWBytes + C::kXBytes));
+            for (int j = 0; j < n; ++j)
+              tma_load_2d(smem_w + (i * kPair + j) * C::kWBytes, &map_w, &full_bar[i], (kb + j) * BLOCK_K, t.w_row0);
+          }
+        }
+        __syncwarp();
+      }
+      pdl_start();
+    }
     for (int vt = blockIdx.x; ok && vt < num_vtiles; vt += gridDim.x) {
       const SwapTile t = get_swap_tile<GROUPED, TN>(vt / split_k, p, m_tiles, n_tiles, tile_start);
       const int split = vt % split_k;
       const int kb_begin = split * kbps, kb_end = min(nkb, kb_begin + kbps);
       for (int kb = kb_begin; kb < kb_end; kb += kPair) {
-        ok = mbar_wait_warp(&done_bar[stage], phase ^ 1u, p.status, 1);
-        if (!ok) break;
+        if (ahead == 0) {
+          ok = mbar_wait_warp(&done_bar[stage], phase ^ 1u, p.status, 1);
+          if (!ok) break;
+        }
         if (elect_one()) {
           const int n = min(kPair, kb_end - kb);
-          mbar_expect_tx(&full_bar[stage], n * (C::kWBytes + C::kXBytes));
+          if (ahead == 0) mbar_expect_tx(&full_bar[stage], n * (C::kWBytes + C::kXBytes));
           for (int j = 0; j < n; ++j) {
-            tma_load_2d(smem_w + (stage * kPair + j) * C::kWBytes, &map_w, &full_bar[stage], (kb + j) * BLOCK_K,
-                        t.w_row0);
-            tma_load_2d(smem_x + (stage * kPair + j) * C::kXBytes, &map_x, &full_bar[stage], (kb + j) * BLOCK_K,
-                        t.row0);
+            if (ahead == 0)
+              tma_load_2d(smem_w + (stage * kPair + j) * C::kWBytes, &map_w, &full_bar[stage], (kb + j) * BLOCK_K, t.w_row0);
+            tma_load_2d(smem_x + (stage * kPair + j) * C::kXBytes, &map_x, &full_bar[stage], (kb + j) * BLOCK_K, t.row0);
           }
         }
+        if (ahead > 0) --ahead;
         __syncwarp();
         if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
       }
@@ -274,6 +285,7 @@ gemm_block_fp8_swapab_kernel(const __grid_constant__ CUtensorMap map_w, const __
     // form) every token's scales sit in a different sector, so: a slot covers 8 k-blocks (the whole
     // sector of a token, fetched as two 16-byte loads), the loads are issued before the wait for the
     // slot, and two warps take alternate fills.
+    if constexpr (!GROUPED) pdl_wait();
     const int which = warp - C::kStagerWarp;
     const bool row_major_vec = !p.sa_ue8m0 && p.sa_stride_g == 1 && (p.sa_stride_m & 3) == 0 &&
                                (reinterpret_cast<uintptr_t>(p.sa) & 15u) == 0;
@@ -449,7 +461,9 @@ gemm_block_fp8_swapab_kernel(const __grid_constant__ CUtensorMap map_w, const __
       if (ok && split_k == 1) {
         for_each_owned([&](float val, int64_t tok, int n) {
           OutT* dst = out + tok * p.ldo + n;
-          *dst = cvt1(dst, val);
+          OutT v = cvt1(dst, val);
+          if (p.bias) v = cvt1(dst, static_cast<float>(v) + static_cast<float>(static_cast<const OutT*>(p.bias)[n]));
+          *dst = v;
         });
       } else if (ok) {
         for_each_owned([&](float val, int64_t tok, int n) {
@@ -489,8 +503,7 @@ int launch_swap(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& 
   const long long tiles = GROUPED ? (m_tiles + p.num_experts) * n_tiles : m_tiles * n_tiles * p.split_k;
   if (tiles > 0x7fffffffLL) return B200_ERR_TOO_LARGE;   // the kernels count tiles in 32 bits
   const int grid = tiles < sm_count() ? static_cast<int>(tiles) : sm_count();
-  kern<<<grid, C::kThreads, C::kSmemBytes, stream>>>(mw, mx, p);
-  B200_CUDA_TRY(cudaGetLastError());
+  B200_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(C::kThreads), C::kSmemBytes, stream, mw, mx, p));
   return B200_OK;
 }
 

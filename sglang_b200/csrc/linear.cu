@@ -5,7 +5,7 @@
 // allocation, argument check and foreign call per kernel.
 #include <algorithm>
 
-#include "common.cuh"
+#include "gemm_common.cuh"
 
 namespace b200 {
 
@@ -39,6 +39,7 @@ struct Arena {
 template <typename T>
 __global__ void __launch_bounds__(256) bias_add_kernel(T* __restrict__ out, const T* __restrict__ bias, int64_t M, int N,
                                                        int64_t ldo) {
+  pdl_start();
   const int n2 = N >> 1;
   const int64_t total = M * n2;
   for (int64_t i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
@@ -54,16 +55,20 @@ int bias_add(void* out, const void* bias, int64_t M, int64_t N, int64_t ldo, int
   if (N % 2 != 0) return B200_ERR_BAD_SHAPE;
   const int64_t blocks = std::min<int64_t>((M * (N / 2) + 255) / 256, 16LL * sm_count());
   if (dtype == B200_DT_BF16)
-    bias_add_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<__nv_bfloat16*>(out),
+    launch_pdl(bias_add_kernel<__nv_bfloat16>, static_cast<unsigned>(blocks), 256, 0, st, static_cast<__nv_bfloat16*>(out),
                                                                    static_cast<const __nv_bfloat16*>(bias), M,
                                                                    static_cast<int>(N), ldo);
   else
-    bias_add_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<__half*>(out),
+    launch_pdl(bias_add_kernel<__half>, static_cast<unsigned>(blocks), 256, 0, st, static_cast<__half*>(out),
                                                                    static_cast<const __half*>(bias), M,
                                                                    static_cast<int>(N), ldo);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
 }
+
+// Up to this many tokens a power-of-two linear takes the weight-streaming kernel as well (its exponent bytes decoded to fp32
+// scales): the block-scaling kernel's 128-row tiles leave most SMs without a tile there (16 x 7168 x 18432: 73 us).
+inline bool few_tokens(int64_t M) { return M <= 192; }
 
 struct LinearPlan {
   uint8_t* q;
@@ -78,7 +83,7 @@ LinearPlan plan_linear(Arena& a, int64_t M, int64_t N, int64_t K, bool ue8m0) {
   p.q = a.take<uint8_t>(static_cast<size_t>(M) * K);
   p.s_ld = align4(M);
   p.s = a.take<uint32_t>(static_cast<size_t>(p.s_ld) * (ue8m0 ? (groups + 3) / 4 : groups));
-  p.partial_bytes = ue8m0 ? 0 : b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K);
+  p.partial_bytes = !ue8m0 || few_tokens(M) ? b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) : 0;
   p.partial = p.partial_bytes ? a.take<uint8_t>(p.partial_bytes) : nullptr;
   return p;
 }
@@ -108,23 +113,22 @@ extern "C" int b200_fp8_linear(const void* x, int dtype, const void* w, int64_t 
   const LinearPlan p = plan_linear(a, M, N, K, scale_mode != 0);
   if (workspace_bytes < a.used) return B200_ERR_TOO_LARGE;
   int rc;
-  if (scale_mode == 0) {
-    float* s = static_cast<float*>(p.s);
-    rc = b200_per_token_group_quant_fp8(x, dtype, p.q, s, M, K, 128, 1, p.s_ld, kQuantEps, -kFp8Max, kFp8Max, stream);
-    if (rc != B200_OK) return rc;
-    rc = b200_fp8_blockwise_scaled_mm_splitk(p.q, K, w, ldw, s, 1, p.s_ld, ws, ws_stride_n, ws_stride_g, out, ldo, dtype,
-                                             M, N, K, 0, p.partial, p.partial_bytes, stream);
-  } else {
-    uint32_t* s = static_cast<uint32_t*>(p.s);
-    rc = b200_per_token_group_quant_fp8_ue8m0(x, dtype, p.q, s, M, K, p.s_ld, kQuantEps, -kFp8Max, kFp8Max, stream);
-    if (rc != B200_OK) return rc;
-    rc = scale_mode == 2 ? b200_fp8_blockwise_scaled_mm_pow2(p.q, K, w, ldw, s, 1, p.s_ld, ws, ws_stride_n, ws_stride_g,
-                                                             out, ldo, dtype, M, N, K, stream)
-                         : b200_fp8_blockwise_scaled_mm_ue8m0(p.q, K, w, ldw, s, 1, p.s_ld, ws, ws_stride_n, ws_stride_g,
-                                                              out, ldo, dtype, M, N, K, stream);
-  }
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (scale_mode == 0)
+    rc = b200_per_token_group_quant_fp8(x, dtype, p.q, static_cast<float*>(p.s), M, K, 128, 1, p.s_ld, kQuantEps, -kFp8Max,
+                                        kFp8Max, stream);
+  else
+    rc = b200_per_token_group_quant_fp8_ue8m0(x, dtype, p.q, static_cast<uint32_t*>(p.s), M, K, p.s_ld, kQuantEps, -kFp8Max,
+                                              kFp8Max, stream);
   if (rc != B200_OK) return rc;
-  return bias ? bias_add(out, bias, M, N, ldo, dtype, static_cast<cudaStream_t>(stream)) : B200_OK;
+  if (scale_mode == 2 && !few_tokens(M)) {
+    rc = b200_fp8_blockwise_scaled_mm_pow2(p.q, K, w, ldw, static_cast<uint32_t*>(p.s), 1, p.s_ld, ws, ws_stride_n,
+                                           ws_stride_g, out, ldo, dtype, M, N, K, stream);
+    return rc == B200_OK && bias ? bias_add(out, bias, M, N, ldo, dtype, st) : rc;
+  }
+  // the kernel before is the quantiser launched above: weights may be fetched while it runs
+  return dense_mm(p.q, K, w, ldw, static_cast<const float*>(p.s), 1, p.s_ld, ws, ws_stride_n, ws_stride_g, out, ldo, dtype,
+                  M, N, K, 0, p.partial, p.partial_bytes, stream, scale_mode != 0, bias, 1);
 }
 
 namespace b200 {

@@ -27,6 +27,7 @@ constexpr int kPrepChunk = 2048;   // ids per chunk
 // ---- phase 1: per-chunk histogram -> scratch[chunk][E]
 __global__ void __launch_bounds__(kPrepThreads)
 prep_count_kernel(const int32_t* __restrict__ topk_ids, int64_t n_ids, int num_experts, int32_t* __restrict__ scratch) {
+  pdl_start();
   extern __shared__ int32_t s_cnt[];
   for (int e = threadIdx.x; e < num_experts; e += kPrepThreads) s_cnt[e] = 0;
   __syncthreads();
@@ -49,6 +50,7 @@ __global__ void __launch_bounds__(1024)
 prep_scan_kernel(int32_t* __restrict__ scratch, int num_chunks, int num_experts, int32_t* __restrict__ expert_offsets,
                  int32_t* __restrict__ blockscale_offsets, int32_t* __restrict__ problem_sizes1,
                  int32_t* __restrict__ problem_sizes2, int n, int k) {
+  pdl_start();
   extern __shared__ int32_t s_tot[];   // [num_experts] totals, then exclusive offsets
   for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
     int run = 0;
@@ -91,6 +93,7 @@ __global__ void __launch_bounds__(kPrepThreads)
 prep_scatter_kernel(const int32_t* __restrict__ topk_ids, int64_t n_ids, int topk, int num_experts,
                     const int32_t* __restrict__ scratch, int32_t* __restrict__ input_permutation,
                     int32_t* __restrict__ output_permutation, int walk_warps) {
+  pdl_start();
   extern __shared__ int32_t s_mem[];
   int32_t* s_ids = s_mem;                          // [kPrepChunk]
   int32_t* s_wnext = s_mem + kPrepChunk;           // [walk_warps][E] next free slot of each expert for each walking warp
@@ -153,6 +156,7 @@ template <typename V>
 __global__ void __launch_bounds__(256)
 rows_gather_kernel(const V* __restrict__ in, const int32_t* __restrict__ map, V* __restrict__ out,
                    int64_t num_dst_rows, int vec_per_row) {
+  pdl_start();
   const int rows_per_block = 256 / 32;   // one warp per row
   const int64_t row = static_cast<int64_t>(blockIdx.x) * rows_per_block + (threadIdx.x >> 5);
   if (row >= num_dst_rows) return;
@@ -201,6 +205,7 @@ struct Pack8<__half> {
 template <typename T>
 __global__ void __launch_bounds__(256)
 silu_and_mul_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t rows, int d) {
+  pdl_start();
   const int vec_per_row = d / 8;
   const int64_t total = rows * vec_per_row;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; i < total;
@@ -224,6 +229,7 @@ template <typename T, typename F>
 __global__ void __launch_bounds__(256)
 unpermute_sum_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __restrict__ perm,
                      const F* __restrict__ factors, int m, int topk, int row_len) {
+  pdl_start();
   const int i = blockIdx.x;
   if (i >= m) return;
   const int vec_per_row = row_len / 8;
@@ -257,15 +263,15 @@ int moe_prepare_launch(const int32_t* topk_ids, int64_t n_ids, int topk, int num
                        int32_t* scratch, cudaStream_t st) {
   const int chunks = static_cast<int>((n_ids + kPrepChunk - 1) / kPrepChunk);
   const int nch = chunks < 1 ? 1 : chunks;
-  prep_count_kernel<<<nch, kPrepThreads, num_experts * sizeof(int32_t), st>>>(topk_ids, n_ids, num_experts, scratch);
-  prep_scan_kernel<<<1, 1024, num_experts * sizeof(int32_t), st>>>(scratch, nch, num_experts, expert_offsets,
+  launch_pdl(prep_count_kernel, nch, kPrepThreads, num_experts * sizeof(int32_t), st, topk_ids, n_ids, num_experts, scratch);
+  launch_pdl(prep_scan_kernel, 1, 1024, num_experts * sizeof(int32_t), st, scratch, nch, num_experts, expert_offsets,
                                                                    blockscale_offsets, problem_sizes1,
                                                                    problem_sizes2, n, k);
   // walking warps: as many (a power of two up to 8) as fit their per-expert tables into 48 KB of shared memory
   int walk_warps = 8;
   while (walk_warps > 1 && (static_cast<size_t>(walk_warps) * num_experts + kPrepChunk) * sizeof(int32_t) > 48 * 1024)
     walk_warps >>= 1;
-  prep_scatter_kernel<<<nch, kPrepThreads, (static_cast<size_t>(walk_warps) * num_experts + kPrepChunk) * sizeof(int32_t), st>>>(
+  launch_pdl(prep_scatter_kernel, nch, kPrepThreads, (static_cast<size_t>(walk_warps) * num_experts + kPrepChunk) * sizeof(int32_t), st, 
       topk_ids, n_ids, topk, num_experts, scratch, input_permutation, output_permutation, walk_warps);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
@@ -359,6 +365,7 @@ __global__ void __launch_bounds__(256) packed_scales_gather_kernel(const uint32_
                                                                     int64_t src_rows, const int32_t* __restrict__ map,
                                                                     uint32_t* __restrict__ dst, int64_t dst_ld,
                                                                     int64_t num_dst_rows) {
+  pdl_start();
   const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (r >= num_dst_rows) return;
   const int64_t c = min(max(static_cast<int64_t>(__ldg(map + r)), int64_t(0)), src_rows - 1);
@@ -378,8 +385,8 @@ extern "C" int b200_shuffle_packed_scales(const uint32_t* input, int64_t input_s
   if (input_stride_pack < num_src_rows || output_stride_pack < num_dst_rows) return B200_ERR_BAD_STRIDE;
   const int64_t blocks = (num_dst_rows + 255) / 256;
   if (blocks > 0x7fffffffLL || words_per_row > 65535) return B200_ERR_TOO_LARGE;
-  packed_scales_gather_kernel<<<dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(words_per_row)), 256, 0,
-                                static_cast<cudaStream_t>(stream)>>>(input, input_stride_pack, num_src_rows, dst2src_map,
+  launch_pdl(packed_scales_gather_kernel, dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(words_per_row)), 256, 0,
+                                static_cast<cudaStream_t>(stream), input, input_stride_pack, num_src_rows, dst2src_map,
                                                                      output, output_stride_pack, num_dst_rows);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
@@ -400,19 +407,19 @@ extern "C" int b200_shuffle_rows(const void* input, const int32_t* dst2src_map, 
   const unsigned grid = static_cast<unsigned>(blocks);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if ((bits & 15u) == 0) {
-    rows_gather_kernel<uint4><<<grid, 256, 0, st>>>(static_cast<const uint4*>(input), dst2src_map,
+    launch_pdl(rows_gather_kernel<uint4>, grid, 256, 0, st, static_cast<const uint4*>(input), dst2src_map,
                                                     static_cast<uint4*>(output), num_dst_rows,
                                                     static_cast<int>(row_bytes / 16));
   } else if ((bits & 7u) == 0) {
-    rows_gather_kernel<uint2><<<grid, 256, 0, st>>>(static_cast<const uint2*>(input), dst2src_map,
+    launch_pdl(rows_gather_kernel<uint2>, grid, 256, 0, st, static_cast<const uint2*>(input), dst2src_map,
                                                     static_cast<uint2*>(output), num_dst_rows,
                                                     static_cast<int>(row_bytes / 8));
   } else if ((bits & 3u) == 0) {
-    rows_gather_kernel<uint32_t><<<grid, 256, 0, st>>>(static_cast<const uint32_t*>(input), dst2src_map,
+    launch_pdl(rows_gather_kernel<uint32_t>, grid, 256, 0, st, static_cast<const uint32_t*>(input), dst2src_map,
                                                        static_cast<uint32_t*>(output), num_dst_rows,
                                                        static_cast<int>(row_bytes / 4));
   } else {
-    rows_gather_kernel<uint8_t><<<grid, 256, 0, st>>>(static_cast<const uint8_t*>(input), dst2src_map,
+    launch_pdl(rows_gather_kernel<uint8_t>, grid, 256, 0, st, static_cast<const uint8_t*>(input), dst2src_map,
                                                       static_cast<uint8_t*>(output), num_dst_rows,
                                                       static_cast<int>(row_bytes));
   }
@@ -432,10 +439,10 @@ extern "C" int b200_silu_and_mul(const void* x, void* out, int64_t rows, int64_t
   if (blocks > cap) blocks = cap;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == B200_DT_BF16) {
-    silu_and_mul_kernel<__nv_bfloat16><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
+    launch_pdl(silu_and_mul_kernel<__nv_bfloat16>, static_cast<unsigned>(blocks), 256, 0, st, 
         static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out), rows, static_cast<int>(d));
   } else if (dtype == B200_DT_F16) {
-    silu_and_mul_kernel<__half><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
+    launch_pdl(silu_and_mul_kernel<__half>, static_cast<unsigned>(blocks), 256, 0, st, 
         static_cast<const __half*>(x), static_cast<__half*>(out), rows, static_cast<int>(d));
   } else {
     return B200_ERR_BAD_DTYPE;
@@ -459,7 +466,7 @@ int unpermute_sum(const void* input, void* output, const int32_t* permutation, c
   auto go = [&](auto* in) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(in)>>;
     using Factor = std::conditional_t<std::is_void_v<F>, T, F>;
-    unpermute_sum_kernel<T, Factor><<<static_cast<unsigned>(m), threads, 0, st>>>(
+    launch_pdl(unpermute_sum_kernel<T, Factor>, static_cast<unsigned>(m), threads, 0, st, 
         in, static_cast<T*>(output), permutation, static_cast<const Factor*>(factors), static_cast<int>(m),
         static_cast<int>(topk), static_cast<int>(row_len));
   };
@@ -508,6 +515,7 @@ __global__ void __launch_bounds__(128) topk_softmax_kernel(const T* __restrict__
                                                            int32_t* __restrict__ ids, int64_t num_tokens,
                                                            int num_experts, int topk, int64_t logits_stride,
                                                            int renormalize) {
+  pdl_start();
   const int lane = threadIdx.x & 31;
   const int64_t token = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (token >= num_tokens) return;
@@ -571,9 +579,9 @@ int launch_router(const void* logits, float* weights, int32_t* ids, int64_t num_
   const unsigned blocks = static_cast<unsigned>((num_tokens + 3) / 4);
   const T* lp = static_cast<const T*>(logits);
   const int per_lane = (num_experts + 31) / 32;
-  if (per_lane <= 2) topk_softmax_kernel<T, 2><<<blocks, 128, 0, st>>>(lp, weights, ids, num_tokens, num_experts, topk, stride, renormalize);
-  else if (per_lane <= 8) topk_softmax_kernel<T, 8><<<blocks, 128, 0, st>>>(lp, weights, ids, num_tokens, num_experts, topk, stride, renormalize);
-  else topk_softmax_kernel<T, kRouterMaxPerLane><<<blocks, 128, 0, st>>>(lp, weights, ids, num_tokens, num_experts, topk, stride, renormalize);
+  if (per_lane <= 2) launch_pdl(topk_softmax_kernel<T, 2>, blocks, 128, 0, st, lp, weights, ids, num_tokens, num_experts, topk, stride, renormalize);
+  else if (per_lane <= 8) launch_pdl(topk_softmax_kernel<T, 8>, blocks, 128, 0, st, lp, weights, ids, num_tokens, num_experts, topk, stride, renormalize);
+  else launch_pdl(topk_softmax_kernel<T, kRouterMaxPerLane>, blocks, 128, 0, st, lp, weights, ids, num_tokens, num_experts, topk, stride, renormalize);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
 }
@@ -618,6 +626,7 @@ __global__ void __launch_bounds__(128) fused_gate_kernel(const float* __restrict
                                                          int64_t num_tokens, int num_experts, int num_groups,
                                                          int topk_group, int topk_all, int64_t logits_stride,
                                                          int num_shared, double routed_scaling_factor) {
+  pdl_start();
   // topk_all output slots per token: the first topk routed choices, then num_shared fused shared experts
   // (ids num_experts, num_experts + 1, ...) whose weight is (sum of the routed scores / routed_scaling_factor)
   // before the common division by that sum (sgl-kernel/csrc/moe/moe_fused_gate.cu:225-252)
@@ -733,11 +742,11 @@ extern "C" int b200_moe_fused_gate_shared_experts(const float* gating_output, in
   const unsigned blocks = static_cast<unsigned>((num_tokens + 3) / 4);
   const size_t smem = 4 * static_cast<size_t>(num_experts) * sizeof(float);
   if (num_experts <= 256)
-    fused_gate_kernel<8><<<blocks, 128, smem, st>>>(gating_output, bias, topk_weights, topk_ids, num_tokens, num_experts,
+    launch_pdl(fused_gate_kernel<8>, blocks, 128, smem, st, gating_output, bias, topk_weights, topk_ids, num_tokens, num_experts,
                                                    num_expert_group, topk_group, topk, row_stride,
                                                    num_fused_shared_experts, routed_scaling_factor);
   else
-    fused_gate_kernel<32><<<blocks, 128, smem, st>>>(gating_output, bias, topk_weights, topk_ids, num_tokens, num_experts,
+    launch_pdl(fused_gate_kernel<32>, blocks, 128, smem, st, gating_output, bias, topk_weights, topk_ids, num_tokens, num_experts,
                                                     num_expert_group, topk_group, topk, row_stride,
                                                     num_fused_shared_experts, routed_scaling_factor);
   B200_CUDA_TRY(cudaGetLastError());

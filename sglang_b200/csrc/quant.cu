@@ -217,6 +217,7 @@ quant_group_kernel(const T* __restrict__ x, const int32_t* __restrict__ src_rows
                    float* __restrict__ s, int64_t M, int64_t K,
                    int64_t s_stride_row, int64_t s_stride_grp, float eps, float fp8_min, float fp8_max,
                    int tiles_k) {
+  pdl_start();
   constexpr int TPG = GROUP / kVec;              // lanes cooperating on one group
   constexpr int GPT = kTileW / GROUP;            // groups per tile row
   constexpr int SLOTS_PER_ROW = kTileW / kVec;   // 64 threads per tile row
@@ -334,6 +335,7 @@ __global__ void __launch_bounds__(kThreads, NV <= 2 ? (HAS_RES ? 4 : 5) : 2) rms
                                                                     int64_t K, int64_t s_stride_row, int64_t s_stride_grp,
                                                                     float norm_eps, float eps, float fp8_min,
                                                                     float fp8_max) {
+  pdl_start();
   __shared__ float red[kThreads / 32];
   const int tid = threadIdx.x;
   const int64_t row = blockIdx.x;
@@ -436,7 +438,7 @@ int launch_group(const void* x, void* q, float* s, int64_t M, int64_t K, int64_t
   const T* xp = static_cast<const T*>(x);
   uint8_t* qp = static_cast<uint8_t*>(q);
 #define B200_LAUNCH_Q(P)                                                                                       \
-  quant_group_kernel<T, GROUP, P, IEEE_DIV, FUSE_SILU, UE8M0, INT8><<<grid, kThreads, 0, stream>>>(xp, src_rows, x_rows, qp, s, M, K, ssr, ssg, eps, fmin_, \
+  launch_pdl(quant_group_kernel<T, GROUP, P, IEEE_DIV, FUSE_SILU, UE8M0, INT8>, grid, kThreads, 0, stream, xp, src_rows, x_rows, qp, s, M, K, ssr, ssg, eps, fmin_, \
                                                                            fmax_, tiles_k)
   switch (passes) {
     case 8:
@@ -654,7 +656,7 @@ extern "C" int b200_rmsnorm_per_token_group_quant_fp8(const void* x, int x_dtype
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const dim3 grid(static_cast<unsigned>(M));
 #define B200_NORM_GO(T, NV, WQ, UE, RES)                                                                              \
-  rmsnorm_quant_kernel<T, WQ, UE, NV, RES><<<grid, kThreads, 0, st>>>(                                                \
+  launch_pdl(rmsnorm_quant_kernel<T, WQ, UE, NV, RES>, grid, kThreads, 0, st, \
       static_cast<const T*>(x), static_cast<T*>(residual), static_cast<const T*>(weight), static_cast<T*>(y),         \
       static_cast<uint8_t*>(q), static_cast<float*>(s), M, K, s_stride_row, s_stride_grp, norm_eps, eps, fp8_min,     \
       fp8_max)
