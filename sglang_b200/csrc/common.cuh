@@ -40,9 +40,11 @@ int require_sm100();
 // Launch with programmatic stream serialisation: the kernel may become resident while the one before it in the stream
 // still runs.  Such a kernel calls pdl_wait() before it touches global memory (the wait ends when everything earlier in
 // the stream has completed and is visible), so results do not depend on the overlap; it hides the launch gap and the
-// kernel's own prologue, 1-3 us per kernel, which is most of a decode-size call.
+// kernel's own prologue, 1-3 us per kernel, which is most of a decode-size call.  A persistent GEMM with several waves of
+// tiles is launched plainly (overlap = false): its CTAs, started one by one as SMs become free, lose the lockstep that
+// keeps the tiles they share in L2, which cost 2-3 % of a multi-millisecond MLP.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+inline cudaError_t launch_overlap(bool overlap, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -52,8 +54,12 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_overlap(true, kern, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 #endif
 
@@ -69,6 +75,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // (weights, in a chain this library launches) was complete before this kernel began.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A persistent kernel with more than one wave of work does not trigger early: its next kernel has little to gain.
+__device__ __forceinline__ void pdl_trigger_if(bool single_wave) {
+  if (single_wave) pdl_trigger();
+}
 __device__ __forceinline__ void pdl_start() {
   pdl_wait();
   pdl_trigger();

@@ -164,7 +164,7 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const int nkb = (p.K + BLOCK_K - 1) / BLOCK_K;
 
   if constexpr (GROUPED) {
-    pdl_start();     // the tables come from the kernels before this one
+    pdl_wait();     // the tables come from the kernels before this one
     build_tile_table(tile_m_start, p.problem_sizes, p.num_experts, TILE_M);
   }
 
@@ -224,8 +224,9 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         }
         __syncwarp();
       }
-      pdl_start();
+      pdl_wait();
     }
+    pdl_trigger_if(num_vtiles <= static_cast<int>(gridDim.x));
     for (int vt = blockIdx.x; ok && vt < num_vtiles; vt += gridDim.x) {
       const Work w = decode_work(vt, p, nkb, GROUPED);
       const TileInfo t = get_tile<GROUPED>(w.tile, p, m_blocks, n_blocks, tile_m_start);
@@ -590,7 +591,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, cu
                                   : split_from + (dense_tiles - split_from) * p.split_k;
   if (tiles > 0x7fffffffLL) return B200_ERR_TOO_LARGE;   // the kernels count tiles in 32 bits
   const int grid = tiles < sm_count() ? static_cast<int>(tiles) : sm_count();
-  B200_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(kThreads), kSmemBytes, stream, ma, mb, p));
+  B200_CUDA_TRY(launch_overlap(tiles <= sm_count(), kern, dim3(grid), dim3(kThreads), kSmemBytes, stream, ma, mb, p));
   return B200_OK;
 }
 

@@ -225,7 +225,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __shared__ float amax_x[SILU_Q ? 2 : 1][2][SILU_Q ? BM : 1];   // fused-activation epilogue: maxima of the two column halves
   __shared__ uint64_t xbar[4];                                    // ... and where the two warps of a row quadrant meet
   if constexpr (GROUPED) {
-    pdl_start();     // the tables come from the kernels before this one
+    pdl_wait();     // the tables come from the kernels before this one
     // row tiles per problem (none for an empty problem or one whose weight slice does not exist) ...
     for (int i = threadIdx.x; i < p.num_problems; i += blockDim.x) {
       const int rows = p.rows ? __ldg(p.rows + static_cast<int64_t>(i) * p.rows_stride) : p.M;
@@ -281,7 +281,8 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
-  if constexpr (!GROUPED) pdl_start();
+  if constexpr (!GROUPED) pdl_wait();
+  pdl_trigger_if(num_tiles <= static_cast<int>(gridDim.x));
 
   if (warp == 4) {
     // ------------------------------------------------------------------ TMA producer
@@ -626,6 +627,12 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
+// Whether a launch may overlap its predecessor (see launch_overlap): one wave of tiles, or -- where the tile count lives on
+// the device -- problems of few rows.
+inline bool short_problem(const MxParams& p, long long tiles) {
+  return p.rows ? p.M <= 64LL * p.num_problems : tiles <= sm_count();
+}
+
 template <int BN, int MSUB, bool GROUPED, typename OutT>
 int launch_mx(const CUtensorMap& ma, const CUtensorMap& mb, const MxParams& p, cudaStream_t stream) {
   using C = MxCfg<BN, MSUB>;
@@ -642,7 +649,7 @@ int launch_mx(const CUtensorMap& ma, const CUtensorMap& mb, const MxParams& p, c
   const long long tiles = m_tiles * ((p.N + BN - 1) / BN);
   if (tiles > 0x7fffffffLL) return B200_ERR_TOO_LARGE;   // the kernels count tiles in 32 bits
   const int grid = tiles < sm_count() ? static_cast<int>(tiles) : sm_count();
-  B200_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3((BN == 256 && MSUB == 1) ? kThreadsMxSilu : kThreadsMx), C::kSmem, stream, ma, mb, p));
+  B200_CUDA_TRY(launch_overlap(short_problem(p, tiles), kern, dim3(grid), dim3((BN == 256 && MSUB == 1) ? kThreadsMxSilu : kThreadsMx), C::kSmem, stream, ma, mb, p));
   return B200_OK;
 }
 
@@ -681,7 +688,7 @@ int launch_mx_silu(const void* a, int64_t lda, const void* b, int64_t ldb, const
   const long long tiles = m_tiles * ((p.N + 127) / 128);
   if (tiles > 0x7fffffffLL) return B200_ERR_TOO_LARGE;   // the kernels count tiles in 32 bits
   const int grid = tiles < sm_count() ? static_cast<int>(tiles) : sm_count();
-  B200_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(kThreadsMxSilu), C::kSmem, stream, ma, mb, p));
+  B200_CUDA_TRY(launch_overlap(short_problem(p, tiles), kern, dim3(grid), dim3(kThreadsMxSilu), C::kSmem, stream, ma, mb, p));
   return B200_OK;
 }
 
@@ -812,7 +819,8 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
-  pdl_start();
+  pdl_wait();
+  pdl_trigger_if(num_tiles <= num_pairs);
 
   if (warp == 4) {
     // ------------------------------------------------------------------ TMA producer (each CTA)
@@ -1044,7 +1052,7 @@ int launch_mx_pair(const CUtensorMap& ma, const CUtensorMap& mb, const MxParams&
   if (pairs > max_pairs[dev]) pairs = max_pairs[dev];
   if (tiles < pairs) pairs = static_cast<int>(tiles);
   cfg.gridDim = dim3(2 * pairs);
-  cfg.numAttrs = 2;
+  cfg.numAttrs = tiles <= pairs ? 2 : 1;
   B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ma, mb, p));
   return B200_OK;
 }

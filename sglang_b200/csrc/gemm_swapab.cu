@@ -151,7 +151,7 @@ gemm_block_fp8_swapab_kernel(const __grid_constant__ CUtensorMap map_w, const __
   const int nkb = (p.K + BLOCK_K - 1) / BLOCK_K;
 
   if constexpr (GROUPED) {
-    pdl_start();     // the tables come from the kernels before this one
+    pdl_wait();     // the tables come from the kernels before this one
     build_tile_table(tile_start, p.problem_sizes, p.num_experts, TN);
   }
   if (threadIdx.x == 0) {
@@ -208,8 +208,9 @@ gemm_block_fp8_swapab_kernel(const __grid_constant__ CUtensorMap map_w, const __
         }
         __syncwarp();
       }
-      pdl_start();
+      pdl_wait();
     }
+    pdl_trigger_if(num_vtiles <= static_cast<int>(gridDim.x));
     for (int vt = blockIdx.x; ok && vt < num_vtiles; vt += gridDim.x) {
       const SwapTile t = get_swap_tile<GROUPED, TN>(vt / split_k, p, m_tiles, n_tiles, tile_start);
       const int split = vt % split_k;
@@ -503,7 +504,7 @@ int launch_swap(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& 
   const long long tiles = GROUPED ? (m_tiles + p.num_experts) * n_tiles : m_tiles * n_tiles * p.split_k;
   if (tiles > 0x7fffffffLL) return B200_ERR_TOO_LARGE;   // the kernels count tiles in 32 bits
   const int grid = tiles < sm_count() ? static_cast<int>(tiles) : sm_count();
-  B200_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(C::kThreads), C::kSmemBytes, stream, mw, mx, p));
+  B200_CUDA_TRY(launch_overlap(GROUPED || tiles <= 2 * sm_count(), kern, dim3(grid), dim3(C::kThreads), C::kSmemBytes, stream, mw, mx, p));
   return B200_OK;
 }
 
