@@ -913,11 +913,13 @@ extern "C" int b200_fp8_blockwise_scaled_grouped_mm(const void* a, int64_t lda, 
 
   // An expert's weights are rows [e*N, (e+1)*N) of one [E*N, K] matrix.
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // Up to 64 rows per expert on average the weight-streaming kernel is used (measured on the DeepSeek-V3
-  // expert shapes, 256 experts: 1.25x at 16-32 rows per expert, level at 64); beyond that an expert fills most
-  // of a 128-row token tile and the wider MMAs of this file's kernel win (1.15x at 96 rows, level at 128).
+  // Up to 56 rows per expert on average the weight-streaming kernel is used: measured on 64 experts of [4096, 7168] it takes
+  // 293 us against 316 at 40 rows, the same at 56 and 444 against 325 at 80.  (Two ways to spare experts of 129-190 rows
+  // their second row tile were built and measured at 128 rows, 386 us: tokens on the MMA's N side, 440-500 us -- the
+  // 16-lane tensor-memory loads it needs are 3.3 times slower than the 32-lane ones -- and 192-row x 128-column tiles,
+  // 495 us -- half as many weight bytes in flight per hand-off.)
   const int64_t avg_rows = total_rows / num_experts;
-  const bool auto_swap = g_force_block_n == 0 && avg_rows <= 64;
+  const bool auto_swap = g_force_block_n == 0 && avg_rows <= 56;
   if ((g_force_block_n == 3 || forced_token_tile() != 0 || auto_swap) && N % 128 == 0) {
     int tt = forced_token_tile();
     if (tt == 0) tt = avg_rows <= 20 ? 32 : 64;
