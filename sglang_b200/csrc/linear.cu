@@ -13,6 +13,9 @@ namespace b200 {
 // conversion pass stored)
 int unpermute_sum_f32_factors(const void* input, void* output, const int32_t* permutation, const float* factors, int64_t m,
                               int64_t topk, int64_t row_len, int dtype, cudaStream_t stream);
+// quant.cu: every token quantised once, codes and scales stored to the rows of its experts
+int quant_to_rows(const void* x, int dtype, const int32_t* row_of, int topk, void* q, void* s, int64_t M, int64_t K,
+                  int64_t s_ld, bool ue8m0, cudaStream_t stream);
 
 namespace {
 
@@ -138,8 +141,8 @@ struct ExpertPlan {
   int32_t *offsets, *ps1, *ps2, *a_map, *c_map;
   uint8_t* prep_scratch;
   size_t prep_bytes;
-  uint8_t *a_q, *rep_q, *inter_q, *c1, *c2;
-  uint32_t *a_s, *rep_s, *inter_s;     // fp32 scales or packed exponent words
+  uint8_t *rep_q, *inter_q, *c1, *c2;
+  uint32_t *rep_s, *inter_s;           // fp32 scales or packed exponent words
 };
 
 ExpertPlan plan_experts(Arena& a, int64_t m, int64_t k, int64_t n, int topk, int E, bool ue8m0) {
@@ -152,16 +155,13 @@ ExpertPlan plan_experts(Arena& a, int64_t m, int64_t k, int64_t n, int topk, int
   p.c_map = a.take<int32_t>(R);
   p.prep_bytes = b200_moe_prepare_scratch_bytes(R, E);
   p.prep_scratch = a.take(p.prep_bytes);
-  p.a_q = a.take(m * k);
   p.rep_q = a.take(R * k);
   p.inter_q = a.take(R * n);
   if (ue8m0) {
-    p.a_s = a.take<uint32_t>(align4(m) * ((gk + 3) / 4));
     p.rep_s = a.take<uint32_t>(align4(R) * ((gk + 3) / 4));
     p.inter_s = a.take<uint32_t>(align4(R) * ((gn + 3) / 4));
     p.c1 = nullptr;
   } else {
-    p.a_s = a.take<uint32_t>(m * gk);
     p.rep_s = a.take<uint32_t>(R * gk);
     p.inter_s = a.take<uint32_t>(R * gn);
     p.c1 = a.take(2 * R * 2 * n);
@@ -204,17 +204,13 @@ extern "C" int b200_fused_experts_fp8(const void* x, int dtype, const void* w13,
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t R = m * topk, gk = k / 128, gn = n / 128;
   const int E = num_experts;
-  // slots past the routed rows (masked ids) gather row 0: in bounds, never used
-  B200_CUDA_TRY(cudaMemsetAsync(p.a_map, 0, R * sizeof(int32_t), st));
   int rc = b200_moe_prepare(topk_ids, m, topk, E, static_cast<int>(n), static_cast<int>(k), p.offsets, nullptr, p.ps1,
                             p.ps2, p.a_map, p.c_map, p.prep_scratch, p.prep_bytes, stream);
   if (rc != B200_OK) return rc;
   if (scale_ue8m0) {
-    const int64_t ld_a = align4(m), ld_r = align4(R);
-    const int wk = static_cast<int>((gk + 3) / 4), wn = static_cast<int>((gn + 3) / 4);
-    rc = b200_per_token_group_quant_fp8_ue8m0(x, dtype, p.a_q, p.a_s, m, k, ld_a, kQuantEps, -kFp8Max, kFp8Max, stream);
-    if (rc == B200_OK) rc = b200_shuffle_rows(p.a_q, p.a_map, p.rep_q, R, k, stream);
-    if (rc == B200_OK) rc = b200_shuffle_packed_scales(p.a_s, ld_a, m, p.a_map, p.rep_s, ld_r, R, wk, stream);
+    const int64_t ld_r = align4(R);
+    const int wn = static_cast<int>((gn + 3) / 4);
+    rc = quant_to_rows(x, dtype, p.c_map, topk, p.rep_q, p.rep_s, m, k, ld_r, true, st);
     if (rc != B200_OK) return rc;
     if (gn % 4 != 0) B200_CUDA_TRY(cudaMemsetAsync(p.inter_s + (wn - 1) * ld_r, 0, ld_r * sizeof(uint32_t), st));
     rc = b200_fp8_blockwise_scaled_grouped_mm_pow2_silu_quant(
@@ -224,10 +220,8 @@ extern "C" int b200_fused_experts_fp8(const void* x, int dtype, const void* w13,
       rc = b200_fp8_blockwise_scaled_grouped_mm_pow2(p.inter_q, n, R, w2, n, p.inter_s, 1, ld_r, -1, w2_scale, gk * gn, gn,
                                                      1, p.c2, k, dtype, p.offsets, p.ps1, 3, nullptr, E, E, k, n, stream);
   } else {
-    float *a_s = reinterpret_cast<float*>(p.a_s), *inter_s = reinterpret_cast<float*>(p.inter_s);
-    rc = b200_per_token_group_quant_fp8(x, dtype, p.a_q, a_s, m, k, 128, gk, 1, kQuantEps, -kFp8Max, kFp8Max, stream);
-    if (rc == B200_OK) rc = b200_shuffle_rows(p.a_q, p.a_map, p.rep_q, R, k, stream);
-    if (rc == B200_OK) rc = b200_shuffle_rows(p.a_s, p.a_map, p.rep_s, R, gk * 4, stream);
+    float* inter_s = reinterpret_cast<float*>(p.inter_s);
+    rc = quant_to_rows(x, dtype, p.c_map, topk, p.rep_q, p.rep_s, m, k, 0, false, st);
     if (rc == B200_OK)
       rc = b200_fp8_blockwise_scaled_grouped_mm(p.rep_q, k, w13, k, reinterpret_cast<float*>(p.rep_s), gk, 1, w13_scale,
                                                 2 * gn * gk, gk, 1, p.c1, 2 * n, dtype, p.offsets, p.ps1, E, R, 2 * n, k,

@@ -44,6 +44,97 @@ prep_count_kernel(const int32_t* __restrict__ topk_ids, int64_t n_ids, int num_e
   for (int e = threadIdx.x; e < num_experts; e += kPrepThreads) out[e] = s_cnt[e];
 }
 
+// Exclusive prefix of the experts' counts in place, by one warp; the running sums go to expert_offsets [E + 1] and, rounded
+// up to 128 per expert, to blockscale_offsets.
+__device__ __forceinline__ void expert_prefix(int32_t* s_tot, int num_experts, int32_t* __restrict__ expert_offsets,
+                                              int32_t* __restrict__ blockscale_offsets) {
+  const int lane = threadIdx.x & 31;
+  int carry = 0, carry_rounded = 0;
+  if (lane == 0) {
+    expert_offsets[0] = 0;
+    if (blockscale_offsets) blockscale_offsets[0] = 0;
+  }
+  for (int base = 0; base < num_experts; base += 32) {
+    const int e = base + lane;
+    const int c = e < num_experts ? s_tot[e] : 0;
+    int v = c, w = (c + 127) / 128 * 128;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, off), x = __shfl_up_sync(0xffffffffu, w, off);
+      if (lane >= off) { v += u; w += x; }
+    }
+    if (e < num_experts) {
+      s_tot[e] = carry + v - c;
+      expert_offsets[e + 1] = carry + v;
+      if (blockscale_offsets) blockscale_offsets[e + 1] = carry_rounded + w;
+    }
+    carry += __shfl_sync(0xffffffffu, v, 31);
+    carry_rounded += __shfl_sync(0xffffffffu, w, 31);
+  }
+}
+
+// ---- all three phases in one block, for id lists that fit: per-warp histograms of contiguous segments, prefix over
+// experts, in-order walk.  A decode batch's tables cost one launch instead of three.  The limit is where one block's walk
+// (n_ids / 32 warps, a few instructions per 32 ids) would take longer than the two launches it saves.
+constexpr int kPrepOneIds = 4096;
+__global__ void __launch_bounds__(1024)
+prep_one_kernel(const int32_t* __restrict__ topk_ids, int n_ids, int topk, int num_experts, int32_t* __restrict__ expert_offsets,
+                int32_t* __restrict__ blockscale_offsets, int32_t* __restrict__ problem_sizes1,
+                int32_t* __restrict__ problem_sizes2, int32_t* __restrict__ input_permutation,
+                int32_t* __restrict__ output_permutation, int n, int k, int walkers) {
+  pdl_start();
+  extern __shared__ int32_t s_one[];
+  int32_t* s_tot = s_one;                        // [E]
+  int32_t* s_next = s_one + num_experts;         // [walkers][E]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int seg = ((n_ids + walkers - 1) / walkers + 31) & ~31;     // ids per walking warp
+  const int lo = warp * seg, hi = min(n_ids, lo + seg);
+  for (int i = threadIdx.x; i < walkers * num_experts; i += blockDim.x) s_next[i] = 0;
+  __syncthreads();
+  if (warp < walkers)
+    for (int i = lo + lane; i < hi; i += 32) {
+      const int e = topk_ids[i];
+      if (e >= 0 && e < num_experts) atomicAdd(&s_next[warp * num_experts + e], 1);
+    }
+  __syncthreads();
+  for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
+    int run = 0;
+    for (int w = 0; w < walkers; ++w) {
+      const int c = s_next[w * num_experts + e];
+      s_next[w * num_experts + e] = run;
+      run += c;
+    }
+    s_tot[e] = run;
+    problem_sizes1[e * 3 + 0] = run;
+    problem_sizes1[e * 3 + 1] = 2 * n;
+    problem_sizes1[e * 3 + 2] = k;
+    problem_sizes2[e * 3 + 0] = run;
+    problem_sizes2[e * 3 + 1] = k;
+    problem_sizes2[e * 3 + 2] = n;
+  }
+  __syncthreads();
+  if (warp == 0) expert_prefix(s_tot, num_experts, expert_offsets, blockscale_offsets);
+  __syncthreads();
+  if (warp >= walkers) return;
+  int32_t* my_next = s_next + warp * num_experts;
+  for (int i0 = lo; i0 < hi; i0 += 32) {
+    const int i = i0 + lane;
+    const int e = i < hi ? topk_ids[i] : -1;
+    const bool valid = e >= 0 && e < num_experts;
+    const unsigned peers = __match_any_sync(0xffffffffu, valid ? e : -1 - lane);
+    if (valid) {
+      const int slot = s_tot[e] + my_next[e] + __popc(peers & ((1u << lane) - 1u));
+      input_permutation[slot] = i / topk;
+      output_permutation[i] = slot;
+    } else if (i < hi) {
+      output_permutation[i] = -1;
+    }
+    __syncwarp();
+    if (valid && (peers >> lane) <= 1u) my_next[e] += __popc(peers);   // highest lane of each group
+    __syncwarp();
+  }
+}
+
 // ---- phase 2 (one block): per expert, exclusive scan over chunks; expert totals -> offsets, sizes.
 // After it, scratch[chunk][e] = first slot (global) of expert e's ids that live in `chunk`.
 __global__ void __launch_bounds__(1024)
@@ -68,19 +159,8 @@ prep_scan_kernel(int32_t* __restrict__ scratch, int num_chunks, int num_experts,
     problem_sizes2[e * 3 + 2] = n;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {   // E is a few hundred at most: a serial prefix is a few microseconds
-    int run = 0, run_rounded = 0;
-    expert_offsets[0] = 0;
-    if (blockscale_offsets) blockscale_offsets[0] = 0;
-    for (int e = 0; e < num_experts; ++e) {
-      const int c = s_tot[e];
-      s_tot[e] = run;
-      run += c;
-      run_rounded += (c + 127) / 128 * 128;
-      expert_offsets[e + 1] = run;
-      if (blockscale_offsets) blockscale_offsets[e + 1] = run_rounded;
-    }
-  }
+  if (threadIdx.x < 32)   // (a serial prefix over 256 experts took 4 us, as long as a small layer's product)
+    expert_prefix(s_tot, num_experts, expert_offsets, blockscale_offsets);
   __syncthreads();
   for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
     const int off = s_tot[e];
@@ -224,30 +304,39 @@ silu_and_mul_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t rows, 
 }
 
 // ---- out[i] = sum_j factors[i*topk+j] * in[perm[i*topk+j]], j ascending, fp32 accumulate
-// (factors in T, or in fp32: rounded to T before use)
+// (factors in T, or in fp32: rounded to T before use).  A block takes one row and blockDim.x vectors of it, and requests
+// up to eight of the row's sources before it adds the first: one row per block with one load in flight per thread left a
+// 16-token layer at 19 us.
 template <typename T, typename F>
 __global__ void __launch_bounds__(256)
 unpermute_sum_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __restrict__ perm,
                      const F* __restrict__ factors, int m, int topk, int row_len) {
   pdl_start();
-  const int i = blockIdx.x;
-  if (i >= m) return;
-  const int vec_per_row = row_len / 8;
-  for (int v = threadIdx.x; v < vec_per_row; v += blockDim.x) {
-    float acc[8];
+  const int vec_per_row = row_len / 8, parts = (vec_per_row + blockDim.x - 1) / blockDim.x;
+  const int i = blockIdx.x / parts, v = (blockIdx.x - i * parts) * blockDim.x + threadIdx.x;
+  if (v >= vec_per_row) return;
+  float acc[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) acc[k] = 0.f;
-    for (int j = 0; j < topk; ++j) {
-      const int src = perm[i * topk + j];
-      if (src < 0) continue;   // masked expert (expert parallel): contributes nothing
-      const float w = factors ? Pack8<T>::to_float(static_cast<T>(factors[i * topk + j])) : 1.0f;
+  for (int k = 0; k < 8; ++k) acc[k] = 0.f;
+  for (int j0 = 0; j0 < topk; j0 += 8) {
+    uint4 raw[8];
+    int src[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      src[j] = j0 + j < topk ? perm[static_cast<int64_t>(i) * topk + j0 + j] : -1;
+      if (src[j] >= 0) raw[j] = __ldg(reinterpret_cast<const uint4*>(in + static_cast<int64_t>(src[j]) * row_len) + v);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (src[j] < 0) continue;   // masked expert (expert parallel): contributes nothing
+      const float w = factors ? Pack8<T>::to_float(static_cast<T>(factors[static_cast<int64_t>(i) * topk + j0 + j])) : 1.0f;
       float f[8];
-      Pack8<T>::unpack(__ldg(reinterpret_cast<const uint4*>(in + static_cast<int64_t>(src) * row_len) + v), f);
+      Pack8<T>::unpack(raw[j], f);
 #pragma unroll
       for (int k = 0; k < 8; ++k) acc[k] += w * f[k];   // contracted to an fma by nvcc, as the reference's `sum += factor * val` is
     }
-    reinterpret_cast<uint4*>(out + static_cast<int64_t>(i) * row_len)[v] = Pack8<T>::pack(acc);
   }
+  reinterpret_cast<uint4*>(out + static_cast<int64_t>(i) * row_len)[v] = Pack8<T>::pack(acc);
 }
 
 }  // namespace
@@ -263,6 +352,20 @@ int moe_prepare_launch(const int32_t* topk_ids, int64_t n_ids, int topk, int num
                        int32_t* scratch, cudaStream_t st) {
   const int chunks = static_cast<int>((n_ids + kPrepChunk - 1) / kPrepChunk);
   const int nch = chunks < 1 ? 1 : chunks;
+  if (n_ids <= kPrepOneIds) {
+    // walking warps: as many (a power of two up to 32, at least 32 ids each) as fit their tables into 48 KB
+    int walkers = 32;
+    while (walkers > 1 && ((walkers - 1) * 32 >= n_ids ||
+                           (static_cast<size_t>(walkers) + 1) * num_experts * sizeof(int32_t) > 48 * 1024))
+      walkers >>= 1;
+    const size_t smem = (static_cast<size_t>(walkers) + 1) * num_experts * sizeof(int32_t);
+    if (smem <= 48 * 1024) {
+      B200_CUDA_TRY(launch_pdl(prep_one_kernel, 1, 1024, smem, st, topk_ids, static_cast<int>(n_ids), topk, num_experts,
+                               expert_offsets, blockscale_offsets, problem_sizes1, problem_sizes2, input_permutation,
+                               output_permutation, n, k, walkers));
+      return B200_OK;
+    }
+  }
   launch_pdl(prep_count_kernel, nch, kPrepThreads, num_experts * sizeof(int32_t), st, topk_ids, n_ids, num_experts, scratch);
   launch_pdl(prep_scan_kernel, 1, 1024, num_experts * sizeof(int32_t), st, scratch, nch, num_experts, expert_offsets,
                                                                    blockscale_offsets, problem_sizes1,
@@ -463,11 +566,13 @@ int unpermute_sum(const void* input, void* output, const int32_t* permutation, c
   if (m > 0x7fffffffLL) return B200_ERR_TOO_LARGE;
   int threads = static_cast<int>(row_len / 8);
   threads = threads > 256 ? 256 : (threads < 32 ? 32 : (threads + 31) / 32 * 32);
+  const int64_t blocks = m * ((row_len / 8 + threads - 1) / threads);
+  if (blocks > 0x7fffffffLL) return B200_ERR_TOO_LARGE;
   auto go = [&](auto* in) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(in)>>;
     using Factor = std::conditional_t<std::is_void_v<F>, T, F>;
-    launch_pdl(unpermute_sum_kernel<T, Factor>, static_cast<unsigned>(m), threads, 0, st, 
-        in, static_cast<T*>(output), permutation, static_cast<const Factor*>(factors), static_cast<int>(m),
+    launch_pdl(unpermute_sum_kernel<T, Factor>, static_cast<unsigned>(blocks), threads, 0, st, in,
+        static_cast<T*>(output), permutation, static_cast<const Factor*>(factors), static_cast<int>(m),
         static_cast<int>(topk), static_cast<int>(row_len));
   };
   if (dtype == B200_DT_BF16) go(static_cast<const __nv_bfloat16*>(input));
@@ -540,30 +645,36 @@ __global__ void __launch_bounds__(128) topk_softmax_kernel(const T* __restrict__
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
   const float inv = 1.0f / sum;
+  // Selection on unsigned keys (a non-negative float's bits + 1; 0 = padding, taken or NaN): each round is a warp-wide
+  // maximum and, among the lanes that hold it, the lowest expert id -- two reductions instead of a ladder of shuffles.
+  // A lane's own best is kept and only searched again by the lane that was picked.
+  uint32_t key[PER_LANE];
+#pragma unroll
+  for (int i = 0; i < PER_LANE; ++i) key[i] = v[i] >= 0.f ? __float_as_uint(v[i]) + 1u : 0u;
+  uint32_t lane_key = 0;
+  int lane_e = 0x7fffffff;
+  auto search = [&]() {
+    lane_key = 0;
+    lane_e = 0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i)
+      if (key[i] > lane_key) { lane_key = key[i]; lane_e = i * 32 + lane; }   // equal values keep the lower id
+  };
+  search();
   float picked_sum = 0.f;
   float my_w = 0.f;      // lane j keeps the j-th pick (topk <= 32)
   int my_id = 0;
   for (int j = 0; j < topk; ++j) {
-    // lane-local best (value descending, expert id ascending), then the warp's best
-    float best = -1.f;
-    int best_e = 0x7fffffff;
-#pragma unroll
-    for (int i = 0; i < PER_LANE; ++i) {
-      const int e = i * 32 + lane;
-      if (v[i] > best) { best = v[i]; best_e = e; }   // equal values keep the earlier (lower) id
-    }
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-      const int oe = __shfl_xor_sync(0xffffffffu, best_e, off);
-      if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
-    }
-    if ((best_e & 31) == lane) {
+    const uint32_t best_key = __reduce_max_sync(0xffffffffu, lane_key);
+    const int best_e = static_cast<int>(
+        __reduce_min_sync(0xffffffffu, lane_key == best_key ? static_cast<uint32_t>(lane_e) : 0x7fffffffu));
+    if (lane_e == best_e) {
 #pragma unroll
       for (int i = 0; i < PER_LANE; ++i)
-        if (i == (best_e >> 5)) v[i] = -1.f;   // taken
+        if (i == (best_e >> 5)) key[i] = 0;   // taken
+      search();
     }
-    const float w = best * inv;
+    const float w = (best_key == 0 ? -1.f : __uint_as_float(best_key - 1u)) * inv;
     picked_sum += w;
     if (lane == j) { my_w = w; my_id = best_e; }
   }
@@ -651,10 +762,30 @@ __global__ void __launch_bounds__(128) fused_gate_kernel(const float* __restrict
       c[i] = -INFINITY;
     }
   }
+  // Order-preserving unsigned keys of the choice scores (-0 made +0; NaN below everything), so that every maximum below is
+  // one warp reduction; ties go to the lower index.
+  constexpr uint32_t kNone = 0u;
+  auto key_of = [](float x) {
+    const uint32_t b = __float_as_uint(x + 0.f);
+    return x != x ? kNone : (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+  };
+  auto value_of = [](uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); };
+  uint32_t key[PER_LANE];
+#pragma unroll
+  for (int i = 0; i < PER_LANE; ++i) key[i] = key_of(c[i]);
   __syncwarp();
   // lane g: sum of the two largest choice scores of group g
   float gscore = -INFINITY;
-  if (lane < num_groups) {
+  if (group_size == 32) {            // register i of all lanes is group i
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+      if (i >= num_groups) break;
+      const uint32_t k1 = __reduce_max_sync(0xffffffffu, key[i]);
+      const unsigned at = __ballot_sync(0xffffffffu, key[i] == k1);
+      const uint32_t k2 = (at & (at - 1u)) ? k1 : __reduce_max_sync(0xffffffffu, key[i] == k1 ? kNone : key[i]);
+      if (lane == i) gscore = (k1 == kNone ? -INFINITY : value_of(k1)) + (k2 == kNone ? -INFINITY : value_of(k2));
+    }
+  } else if (lane < num_groups) {
     float m1 = -INFINITY, m2 = -INFINITY;
     for (int j = 0; j < group_size; ++j) {
       const float x = choice[lane * group_size + j];
@@ -662,48 +793,49 @@ __global__ void __launch_bounds__(128) fused_gate_kernel(const float* __restrict
     }
     gscore = m1 + m2;
   }
-  // the topk_group best groups -> bit mask
+  // the topk_group best groups -> bit mask (a group whose score is NaN or -inf comes last, in index order)
   uint32_t keep = 0;
+  bool group_left = lane < num_groups;
+  const uint32_t gkey = key_of(gscore);
   for (int j = 0; j < topk_group; ++j) {
-    float best = gscore;
-    int best_g = lane < num_groups ? lane : 0x7fffffff;
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-      const int og = __shfl_xor_sync(0xffffffffu, best_g, off);
-      if (ob > best || (ob == best && og < best_g)) { best = ob; best_g = og; }
-    }
+    const uint32_t best = __reduce_max_sync(0xffffffffu, group_left ? gkey : 0u);
+    const uint32_t best_g = __reduce_min_sync(0xffffffffu, group_left && gkey == best ? static_cast<uint32_t>(lane) : 31u);
     keep |= 1u << best_g;
-    if (lane == best_g) gscore = -INFINITY;
+    if (lane == static_cast<int>(best_g)) group_left = false;
   }
+  constexpr uint32_t kMinusInf = 0x007fffffu;      // the key of -infinity: never picked, like everything at or below it
+  uint32_t lane_key = kMinusInf;
+  int lane_e = 0x7fffffff;
 #pragma unroll
   for (int i = 0; i < PER_LANE; ++i) {
     const int e = i * 32 + lane;
-    if (e < num_experts && !((keep >> (e / group_size)) & 1u)) c[i] = -INFINITY;
+    if (e >= num_experts || !((keep >> (e / group_size)) & 1u)) key[i] = kNone;
   }
+  auto search = [&]() {
+    lane_key = kMinusInf;
+    lane_e = 0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i)
+      if (key[i] > lane_key) { lane_key = key[i]; lane_e = i * 32 + lane; }   // equal values keep the lower id
+  };
+  search();
   float picked_sum = 0.f, my_w = 0.f;
   int my_id = 0;
   for (int j = 0; j < topk; ++j) {
-    float best = -INFINITY;
-    int best_e = 0x7fffffff;
-    float best_s = 0.f;
-#pragma unroll
-    for (int i = 0; i < PER_LANE; ++i) {
-      const int e = i * 32 + lane;
-      if (e < num_experts && c[i] > best) { best = c[i]; best_e = e; best_s = s[i]; }   // equal values keep the lower id
-    }
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-      const int oe = __shfl_xor_sync(0xffffffffu, best_e, off);
-      const float os = __shfl_xor_sync(0xffffffffu, best_s, off);
-      if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; best_s = os; }
-    }
-    if ((best_e & 31) == lane) {
+    const uint32_t best_key = __reduce_max_sync(0xffffffffu, lane_key);
+    const int best_e = static_cast<int>(
+        __reduce_min_sync(0xffffffffu, lane_key == best_key ? static_cast<uint32_t>(lane_e) : 0x7fffffffu));
+    float mine = 0.f;
+    if (lane_e == best_e && best_e != 0x7fffffff) {
 #pragma unroll
       for (int i = 0; i < PER_LANE; ++i)
-        if (i == (best_e >> 5)) c[i] = -INFINITY;   // taken
+        if (i == (best_e >> 5)) {
+          mine = s[i];
+          key[i] = kNone;   // taken
+        }
+      search();
     }
+    const float best_s = __shfl_sync(0xffffffffu, mine, best_e & 31);
     picked_sum += best_s;
     if (lane == j) { my_w = best_s; my_id = best_e; }
   }
