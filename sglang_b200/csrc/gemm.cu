@@ -11,7 +11,7 @@
 // 512 cycles of tensor pipe beside 362 cycles of tensor-memory loads and packed FMAs (each measured alone and together),
 // so the read-out fits under the MMAs as long as nothing makes either side wait.  One persistent CTA per SM, 12 warps:
 //   warps 0-7   promotion + epilogue: each owns 32 rows (its tensor-memory lane quadrant) x half of the tile's columns;
-//               per k-block it reads the partial sums with tcgen05.ld in 32-column chunks, hands the accumulator back
+//               per k-block it reads the partial sums with tcgen05.ld in 64-column chunks, hands the accumulator back
 //               after the last chunk has landed, and does acc += partial * (sa[m,kb] * sb[nb,kb]) with packed FMAs
 //   TMA warp    producer: one A box (128 x 128 B) and one or two B boxes per k-block into a 4-stage ring, 128-byte swizzle
 //   MMA warp    issuer: 4 x tcgen05.mma kind::f8f6f4 (M128 x N256 x K32) per k-block into one of two accumulators, each
@@ -24,7 +24,7 @@
 //   * wait for its scale: products staged by a warp that loads, multiplies and stores one slot at a time paced the kernel
 //     at one slot per global-memory round trip (1300), and a scale fetched where it is used costs its latency (977 -> 863);
 //   * spill: shared memory takes the whole L1, so a spilled register is an L2 round trip.  Eight warps of 128 columns with
-//     184 registers hold the accumulators; sixteen warps of 64 columns (104 registers) spill;
+//     216 registers hold the accumulators and a 64-column chunk; sixteen warps of 64 columns (104 registers) spill;
 //   * write its row in 16-byte pieces (863 -> 803 with 32-byte stores).
 // What bounds it now at large M is power: 803 cycles at the 1.45-1.5 GHz that the chip holds, where the same loop without
 // stores runs 739.  (A CTA pair with two 128-column halves and four accumulators measured 946 cycles without loads or
@@ -54,17 +54,17 @@ constexpr int kEpiWarps = 8;
 constexpr int kTmaWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1, kStagerWarp = kEpiWarps + 2;
 constexpr int kThreads = 32 * (kEpiWarps + 4);
 constexpr int CPW = 128;        // columns per read-out warp: one half of the tile
-constexpr int kChunk = 32;      // columns per tensor-memory round trip
+constexpr int kChunk = 64;      // columns per tensor-memory round trip (32: up to 4 % slower from 512 rows on)
 constexpr int kSlotFloats = TILE_M * kScaleGroup + 2 * kScaleGroup;   // [128 rows][4 k-blocks], then [2 halves][4]
 constexpr int kScaleBytes = kScaleSlots * kSlotFloats * 4;
 constexpr int kMaxExperts = 1024;               // grouped form: m-tile prefix table in shared memory
 constexpr int kSmemBytes = kStages * kStageBytes + kScaleBytes + 1024 /*alignment slack*/ + 512 /*barriers*/;
 static_assert(kSmemBytes + (kMaxExperts + 2) * 4 <= 227 * 1024, "shared memory");
-// The launch gives every thread 168 registers (12 warps); the helper warpgroup hands 32 per thread back and the read-out
-// warps take 16 more each: 128 accumulators, a 32-column chunk and the loop without a spill (168 spills).  setmaxnreg.inc
+// The launch gives every thread 168 registers (12 warps); the helper warpgroup hands 96 per thread back and the read-out
+// warps take 48 more each: 128 accumulators, a 64-column chunk and the loop without a spill (208 spills).  setmaxnreg.inc
 // WAITS until the CTA's pool holds the registers it asks for, so the request must never exceed what the helpers release
 // (the build checks the register count ptxas reports).
-constexpr int kLaunchRegs = 168, kEpiRegs = 184, kHelperRegs = 136;
+constexpr int kLaunchRegs = 168, kEpiRegs = 216, kHelperRegs = 72;
 static_assert(kEpiWarps * (kEpiRegs - kLaunchRegs) <= 4 * (kLaunchRegs - kHelperRegs),
               "read-out warps would wait forever for registers nobody releases");
 
@@ -410,6 +410,7 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           if (ch == 64 && !wide) break;
           float v[kChunk];
           tmem_ld32(taddr + ch, v);
+          tmem_ld32(taddr + ch + 32, v + 32);
           if (ch == 0) {
             sa_v = sa::ld_f32(sc_row + sc_next + (p.sa_ue8m0 ? 0 : jn));
             sb_v = sa::ld_f32(sc_b + sc_next + jn);
@@ -625,12 +626,20 @@ inline int forced_token_tile() {
 namespace b200 {
 namespace {
 
-// Which kernel a dense problem gets: up to 192 tokens the weight-streaming kernel (gemm_swapab.cu,
-// 128 weight rows x up to 64 tokens per tile).  Measured against this file's tiles on the DeepSeek-V3 and
-// Llama-3-70B projections: 10-30 % faster up to 64 tokens, 0-25 % faster for 65-192 (two or three token tiles per
-// weight tile, the second and third reading the weights from L2), slower from 256 on.
-inline bool dense_uses_swapab(int64_t M) { return M <= 192; }
+// Which kernel a dense problem gets.  Up to 64 tokens the weight-streaming kernel (gemm_swapab.cu, 128 weight rows x up to
+// 64 tokens per tile): 0-30 % faster than this file's tiles on every projection.  For 65-192 tokens it has two or three
+// token tiles per weight tile, the second and third reading the weights from L2, and stays ahead (0-25 %) only while all
+// of them run at once; in several waves it re-reads more than it saves.  128 tokens, us, weight-streaming / this file's:
+// [4096, 7168] 14.2 / 16.8 (64 tiles), [8192, 8192] 21.0 / 26.6 (128), [10240, 8192] 35.2 / 28.4 (160),
+// [36864, 7168] 62.1 / 49.6 (576); 192 tokens: [5120, 8192] 19.1 / 29.1 (120), [7168, 9216] 35.9 / 30.7 (168).  With
+// three token tiles two well-filled waves still pass ([10240, 8192], 240 tiles: 33.4 / 35.1).
+constexpr int64_t kStreamTokens = 192;
 inline int dense_token_tile(int64_t M) { return M <= 32 ? 32 : 64; }
+inline bool dense_uses_swapab(int64_t M, int64_t N, int sms) {
+  if (M <= 64 || M > kStreamTokens) return M <= 64;
+  const int64_t tiles = ((M + 63) / 64) * ((N + 127) / 128);
+  return tiles <= sms || (M > 128 && 2 * tiles > 3 * sms && tiles <= 2 * sms);
+}
 
 // Split count for small M (up to 512 rows): when the output has too few tiles for the SMs, the k-blocks of
 // each tile are spread over several CTAs so that the weights stream through all SMs at once.
@@ -638,7 +647,8 @@ int plan_split_k(int64_t M, int64_t N, int64_t K, int sms) {
   if (M > 4 * TILE_M || (N % 4) != 0) return 1;   // beyond 512 rows the tile count is never that small
   const int64_t m_blocks = (M + TILE_M - 1) / TILE_M;
   const int64_t tt = dense_token_tile(M);
-  const int64_t tiles = dense_uses_swapab(M) ? ((M + tt - 1) / tt) * ((N + 127) / 128) : m_blocks * ((N + 255) / 256);
+  const bool stream = M <= kStreamTokens;
+  const int64_t tiles = stream ? ((M + tt - 1) / tt) * ((N + 127) / 128) : m_blocks * ((N + 255) / 256);
   const int64_t nkb = (K + BLOCK_K - 1) / BLOCK_K;
   // measured on DeepSeek-V3 shapes: below 32 k-blocks the launch and pipeline ramp dominate and the
   // extra reduce kernel costs more than the idle SMs
@@ -647,7 +657,7 @@ int plan_split_k(int64_t M, int64_t N, int64_t K, int sms) {
     // More tiles than half the SMs.  The weight-streaming kernel with two or three token tiles per weight tile can
     // still leave most of its last wave empty (DeepSeek-V3 down projection at 129-192 tokens: 168 tiles on 148 SMs;
     // measured 63.9 us unsplit, 55.5 us split in two): split only to fill such a wave.
-    if (!dense_uses_swapab(M)) return 1;
+    if (!stream) return 1;
     auto fill = [sms](int64_t t) { return static_cast<double>(t) / static_cast<double>(((t + sms - 1) / sms) * sms); };
     if (fill(tiles) >= 0.7) return 1;
     for (int s2 = 2; s2 <= 4; ++s2)
@@ -697,8 +707,9 @@ TailPlan plan_tail(int64_t M, int64_t N, int64_t K, int sms) {
 // divided among several CTAs.  A CTA works through the tiles with a fixed stride, so a last wave that fills few of the
 // SMs costs as much as a full one, and a problem of fewer tiles than SMs leaves the rest idle: the k-blocks of just
 // those tiles are spread over the idle SMs, each writing fp32 planes that a second kernel adds in split order.
-// Cost in cycles of the longest CTA: its k-blocks at the measured rate of the tile width, a tile's ramp and epilogue, and
-// for a split the second kernel (2.5 us) and the planes' round trip through L2 (about 4 TB/s).
+// Cost in cycles of the longest CTA: its k-blocks at the measured rate of the tile width (a 128-column k-block costs nearly
+// as much as a 256-column one: the read-out's waits and the way round the pipeline are the same), a tile's ramp and
+// epilogue, and for a split the second kernel (about 5 us) and the planes' round trip through L2 (about 3 TB/s).
 struct TilePlan {
   int tile_n = 256, split_k = 1, kb_per_split = 0, tail_first = 0;
   size_t bytes = 0;
@@ -708,7 +719,7 @@ TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, size_t max_bytes) 
   TilePlan best;
   double best_cost = 0;
   for (const int tile_n : {256, 128}) {
-    const double kb_cycles = tile_n == 256 ? 640.0 : 400.0, tile_cycles = 2500.0;
+    const double kb_cycles = tile_n == 256 ? 850.0 : 720.0, tile_cycles = 2500.0;
     const int64_t tiles = ((M + TILE_M - 1) / TILE_M) * ((N + tile_n - 1) / tile_n);
     const int64_t full = tiles / sms, rest = tiles % sms;
     auto consider = [&](const TilePlan& q, double cost) {
@@ -727,13 +738,21 @@ TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, size_t max_bytes) 
       q.tail_first = static_cast<int>(tiles - rest);
       q.bytes = static_cast<size_t>(rest) * q.split_k * TILE_M * tile_n * sizeof(float);
       if (q.split_k < 2 || q.bytes > max_bytes) continue;
-      consider(q, static_cast<double>(full) * wave + q.kb_per_split * kb_cycles + tile_cycles + 4500.0 + 2.0 * q.bytes / 2300.0);
+      consider(q, static_cast<double>(full) * wave + q.kb_per_split * kb_cycles + tile_cycles + 9000.0 + 2.0 * q.bytes / 1700.0);
     }
   }
   return best;
 }
 
 }  // namespace
+
+// A linear with power-of-two scales on both operands: whether the promoting kernels of this file and gemm_swapab.cu take the product
+// (exponent bytes decoded to fp32 scales) instead of the block-scaling one.  That one has one tile shape per size and no
+// split, so below a few waves of tiles it leaves SMs idle; with enough tiles its MMAs accumulate without read-outs and
+// win.  us, promoting / block-scaling: 16 x 7168 x 18432 29 / 73, 256 x 7168 x 18432 56 / 77, 512 x 10240 x 8192 56 / 71,
+// 768 x 7168 x 18432 101 / 139, 640 x 57344 x 8192 295 / 350, 768 x 36864 x 7168 184 / 178, 1024 x 7168 x 18432 143 / 115,
+// 2048 x 8192 x 8192 140 / 129.
+bool packed_promotes(int64_t M) { return M < 1024; }
 
 int dense_mm(const void* a, int64_t lda, const void* b, int64_t ldb, const float* sa, int64_t sa_stride_m,
              int64_t sa_stride_g, const float* sb, int64_t sb_stride_n, int64_t sb_stride_g, void* out, int64_t ldo,
@@ -759,7 +778,7 @@ int dense_mm(const void* a, int64_t lda, const void* b, int64_t ldb, const float
   if (rc != B200_OK) return rc;
   if (gemm_sticky_status() != 0) return B200_ERR_DEVICE_TIMEOUT;   // sticky until b200_gemm_device_status clears it
   TilePlan plan;
-  const bool swapab = g_force_block_n == 3 || forced_token_tile() != 0 || (g_force_block_n == 0 && dense_uses_swapab(M));
+  const bool swapab = g_force_block_n == 3 || forced_token_tile() != 0 || (g_force_block_n == 0 && dense_uses_swapab(M, N, sm_count()));
   if (!swapab && (split_k == 1 || (split_k == 0 && (!workspace || !aligned16(workspace)))))
     plan = plan_tiles(M, N, K, sm_count(), 0);
   if (split_k == 0) {
@@ -863,7 +882,7 @@ extern "C" int b200_fp8_blockwise_scaled_mm_splitk_plan(int64_t M, int64_t N, in
   const int s = (M == 0 || N == 0) ? 1 : b200::plan_split_k(M, N, K, sms);
   *split_k = s;
   *workspace_bytes = s > 1 ? b200::splitk_workspace_bytes(s, M, N) : 0;
-  if (s == 1 && M > 128 && !b200::dense_uses_swapab(M) && N > 0) {   // large M: split of the last, mostly empty wave of tiles
+  if (s == 1 && M > 128 && M > b200::kStreamTokens && N > 0) {   // large M: split of the last, mostly empty wave of tiles
     const b200::TailPlan t = b200::plan_tail(M, N, K, sms);
     if (t.split_k > 1) {
       *split_k = t.split_k;
@@ -944,7 +963,7 @@ extern "C" int b200_debug_force_block_n(int block_n) {
 extern "C" size_t b200_fp8_blockwise_scaled_mm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (dense_uses_swapab(M)) {
+  if (dense_uses_swapab(M, N, sm_count())) {
     const int s = plan_split_k(M, N, K, sm_count());
     return s > 1 ? splitk_workspace_bytes(s, M, N) : 0;
   }

@@ -54,6 +54,9 @@ int dense_mm(const void* a, int64_t lda, const void* b, int64_t ldb, const float
              int out_dtype, int64_t M, int64_t N, int64_t K, int split_k, void* workspace, size_t workspace_bytes,
              void* stream, int sa_ue8m0, const void* bias, int prefetch_w);
 
+// Whether a linear with power-of-two scales on both sides runs on dense_mm rather than the block-scaling kernel.
+bool packed_promotes(int64_t M);
+
 #if defined(__CUDACC__)
 // Row-tile prefix table of the grouped form, by the whole CTA: per-expert counts, then a warp's running sum.
 __device__ __forceinline__ void build_tile_table(int* tile_start, const int32_t* problem_sizes, int num_experts, int tile_rows) {

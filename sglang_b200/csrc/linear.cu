@@ -69,10 +69,6 @@ int bias_add(void* out, const void* bias, int64_t M, int64_t N, int64_t ldo, int
   return B200_OK;
 }
 
-// Up to this many tokens a power-of-two linear takes the weight-streaming kernel as well (its exponent bytes decoded to fp32
-// scales): the block-scaling kernel's 128-row tiles leave most SMs without a tile there (16 x 7168 x 18432: 73 us).
-inline bool few_tokens(int64_t M) { return M <= 192; }
-
 struct LinearPlan {
   uint8_t* q;
   void* s;
@@ -80,13 +76,14 @@ struct LinearPlan {
   void* partial;
   size_t partial_bytes;
 };
-LinearPlan plan_linear(Arena& a, int64_t M, int64_t N, int64_t K, bool ue8m0) {
+LinearPlan plan_linear(Arena& a, int64_t M, int64_t N, int64_t K, int scale_mode) {
+  const bool ue8m0 = scale_mode != 0;
   LinearPlan p;
   const int64_t groups = K / 128;
   p.q = a.take<uint8_t>(static_cast<size_t>(M) * K);
   p.s_ld = align4(M);
   p.s = a.take<uint32_t>(static_cast<size_t>(p.s_ld) * (ue8m0 ? (groups + 3) / 4 : groups));
-  p.partial_bytes = !ue8m0 || few_tokens(M) ? b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) : 0;
+  p.partial_bytes = scale_mode != 2 || packed_promotes(M) ? b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) : 0;
   p.partial = p.partial_bytes ? a.take<uint8_t>(p.partial_bytes) : nullptr;
   return p;
 }
@@ -98,7 +95,7 @@ extern "C" size_t b200_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t 
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   Arena a(nullptr);
-  plan_linear(a, M, N, K, scale_mode != 0);
+  plan_linear(a, M, N, K, scale_mode);
   return a.used;
 }
 
@@ -113,7 +110,7 @@ extern "C" int b200_fp8_linear(const void* x, int dtype, const void* w, int64_t 
   if (!aligned16(workspace)) return B200_ERR_MISALIGNED;
   if (scale_mode < 0 || scale_mode > 2) return B200_ERR_UNSUPPORTED;
   Arena a(workspace);
-  const LinearPlan p = plan_linear(a, M, N, K, scale_mode != 0);
+  const LinearPlan p = plan_linear(a, M, N, K, scale_mode);
   if (workspace_bytes < a.used) return B200_ERR_TOO_LARGE;
   int rc;
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -124,7 +121,7 @@ extern "C" int b200_fp8_linear(const void* x, int dtype, const void* w, int64_t 
     rc = b200_per_token_group_quant_fp8_ue8m0(x, dtype, p.q, static_cast<uint32_t*>(p.s), M, K, p.s_ld, kQuantEps, -kFp8Max,
                                               kFp8Max, stream);
   if (rc != B200_OK) return rc;
-  if (scale_mode == 2 && !few_tokens(M)) {
+  if (scale_mode == 2 && !packed_promotes(M)) {
     rc = b200_fp8_blockwise_scaled_mm_pow2(p.q, K, w, ldw, static_cast<uint32_t*>(p.s), 1, p.s_ld, ws, ws_stride_n,
                                            ws_stride_g, out, ldo, dtype, M, N, K, stream);
     return rc == B200_OK && bias ? bias_add(out, bias, M, N, ldo, dtype, st) : rc;

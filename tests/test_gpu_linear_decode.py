@@ -29,12 +29,13 @@ def test_decode_linear_matches_the_oracle(M, N, K, dtype):
     assert torch.equal(out, with_bias)
 
 
-@pytest.mark.parametrize("M", [1, 31, 64])
-def test_decode_linear_power_of_two_scales(M):
+@pytest.mark.parametrize("M,N", [(1, 640), (31, 640), (64, 640), (65, 9600), (192, 9600), (193, 640), (512, 1280),
+                                 (513, 1280), (1023, 8192), (1024, 640)])
+def test_decode_linear_power_of_two_scales(M, N):
     from sglang_b200.layers.quantization.fp8_kernel import sglang_per_token_group_quant_fp8, w8a8_block_fp8_matmul_deepgemm
     from sglang_b200.layers.quantization.fp8_utils import (deepgemm_w8a8_block_fp8_linear_with_fallback,
                                                             requant_weight_ue8m0)
-    N, K = 640, 2304
+    K = 2304
     g = torch.Generator(device="cuda").manual_seed(M)
     x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
     wq, ws = O.gen_weight(N, K, seed=9)
@@ -43,3 +44,9 @@ def test_decode_linear_power_of_two_scales(M):
     q, s = sglang_per_token_group_quant_fp8(x, 128, column_major_scales=True, scale_tma_aligned=True, scale_ue8m0=True)
     ref = w8a8_block_fp8_matmul_deepgemm(q, wq, s, ws, [128, 128], torch.bfloat16, weight_scale_ue8m0=True)
     assert O.rel_l2(out.float().cpu(), ref.float().cpu()) <= 1e-3
+    q_f, s_f, w_f = q.float().view(M, -1, 128), s, wq.float().view(N // 128, 128, K // 128, 128)
+    byte = torch.stack([(s_f >> (8 * b)) & 0xff for b in range(4)], dim=-1).reshape(M, -1)[:, :K // 128]
+    a_f = (q_f * torch.exp2(byte.float() - 127).unsqueeze(-1)).view(M, K)
+    b_f = (w_f * ws.view(N // 128, 1, K // 128, 1)).reshape(N, K)
+    exact = (a_f.double() @ b_f.double().T).to(torch.bfloat16)
+    assert O.rel_l2(ref.float().cpu(), exact.float().cpu()) <= 1e-3
