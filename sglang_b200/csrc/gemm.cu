@@ -746,13 +746,20 @@ TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, size_t max_bytes) 
 
 }  // namespace
 
-// A linear with power-of-two scales on both operands: whether the promoting kernels of this file and gemm_swapab.cu take the product
-// (exponent bytes decoded to fp32 scales) instead of the block-scaling one.  That one has one tile shape per size and no
-// split, so below a few waves of tiles it leaves SMs idle; with enough tiles its MMAs accumulate without read-outs and
-// win.  us, promoting / block-scaling: 16 x 7168 x 18432 29 / 73, 256 x 7168 x 18432 56 / 77, 512 x 10240 x 8192 56 / 71,
-// 768 x 7168 x 18432 101 / 139, 640 x 57344 x 8192 295 / 350, 768 x 36864 x 7168 184 / 178, 1024 x 7168 x 18432 143 / 115,
-// 2048 x 8192 x 8192 140 / 129.
-bool packed_promotes(int64_t M) { return M < 1024; }
+// A linear with power-of-two scales on both operands: whether the promoting kernels of this file and gemm_swapab.cu take the
+// product (exponent bytes decoded to fp32 scales) instead of the block-scaling one, which accumulates in tensor memory
+// without read-outs but cannot divide a tile's k-blocks.  us, promoting / block-scaling:
+//   few tiles: 16 x 7168 x 18432 27 / 46, 128 x 8192 x 8192 19.1 / 24.2, 256 x 1280 x 8192 16.0 / 22.9
+//   its 128 x 128 tiles fill more than half of the SMs once: 128 x 10240 x 8192 29.0 / 26.4, 256 x 8192 x 8192 28.2 / 24.7,
+//     512 x 4096 x 7168 25.0 / 22.1 -- up to 64 rows the weight-streaming kernel is still ahead (64 x 10240 x 8192
+//     21.7 / 25.0), and so are its splits at very long K (256 x 8192 x 28672 71.8 / 78.8)
+//   more than one such wave: 640 x 57344 x 8192 295 / 350, 768 x 7168 x 18432 101 / 139, 768 x 36864 x 7168 184 / 178
+//   from 1024 rows on: 1024 x 7168 x 18432 143 / 115, 2048 x 8192 x 8192 140 / 129
+bool packed_promotes(int64_t M, int64_t N, int64_t K) {
+  const int64_t tiles = ((M + 127) / 128) * ((N + 127) / 128);
+  const bool one_full_wave = tiles <= sm_count() && 2 * tiles > sm_count();
+  return M < 1024 && !(one_full_wave && M > 64 && K < 16384);
+}
 
 int dense_mm(const void* a, int64_t lda, const void* b, int64_t ldb, const float* sa, int64_t sa_stride_m,
              int64_t sa_stride_g, const float* sb, int64_t sb_stride_n, int64_t sb_stride_g, void* out, int64_t ldo,

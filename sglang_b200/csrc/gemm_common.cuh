@@ -55,7 +55,7 @@ int dense_mm(const void* a, int64_t lda, const void* b, int64_t ldb, const float
              void* stream, int sa_ue8m0, const void* bias, int prefetch_w);
 
 // Whether a linear with power-of-two scales on both sides runs on dense_mm rather than the block-scaling kernel.
-bool packed_promotes(int64_t M);
+bool packed_promotes(int64_t M, int64_t N, int64_t K);
 
 #if defined(__CUDACC__)
 // Row-tile prefix table of the grouped form, by the whole CTA: per-expert counts, then a warp's running sum.

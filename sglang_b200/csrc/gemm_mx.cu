@@ -39,6 +39,7 @@ constexpr int kGroupMMx = 32;
 
 // Tile shapes (rows x columns per CTA) and their tensor-memory maps:
 //   128 x 256  one accumulator [0,256), scale factors at [256,268).
+//   128 x 128  two accumulators, six stages: few tiles (see the dispatch).
 //   128 x 240  two accumulators [0,240) and [256,496), scale factors at [240,252): a tile's read-out overlaps the
 //              next tile's MMAs.
 //   256 x 240  (MSUB = 2) two 128-row halves that share every B stage: accumulators [0,240) and [256,496), scale
@@ -48,7 +49,7 @@ constexpr int kGroupMMx = 32;
 template <int BN, int MSUB>
 struct MxCfg {
   static_assert(MSUB == 1 || BN <= 240, "two 128-row halves need the 240-wide tile");
-  static constexpr int kStages = MSUB == 2 ? 3 : (BN <= 192 ? 5 : 4);
+  static constexpr int kStages = MSUB == 2 ? 3 : (BN <= 128 ? 6 : (BN <= 192 ? 5 : 4));
   static constexpr int kNumAcc = (BN <= 240 && MSUB == 1) ? 2 : 1;   // accumulator double buffering across tiles
   static constexpr int kABytes = MSUB * BM * BK;
   static constexpr int kBBytes = BN * BK;
@@ -1114,11 +1115,18 @@ extern "C" int b200_fp8_blockwise_scaled_mm_pow2(const void* a, int64_t lda, con
   // (fewer, longer tiles amortise its unoverlapped read-out), wide N with K up to 8192 the CTA pair (half the
   // operand bytes per SM).  With every SM issuing MMAs back to back and nothing else the chip settles at 1.5 GHz
   // under its power cap (3.7 PFLOP/s); these kernels reach 2.5-2.7 and slow down the longer they run.
-  // The test hook selects a form directly: 256 / 240 / 2240 / 2256.
+  // The test hook selects a form directly: 256 / 240 / 2240 / 2256 / 2128.
+  if (g_force_block_n == 2128) return launch_mx_dtype<128, 1>(a, lda, b, ldb, p, st);
   if (g_force_block_n == 2256) return launch_mx_pair_dtype(a, lda, b, ldb, p, st);
   if (g_force_block_n == 256) return launch_mx_dtype<256, 1>(a, lda, b, ldb, p, st);
   if (g_force_block_n == 240) return launch_mx_dtype<240, 1>(a, lda, b, ldb, p, st);
   if (g_force_block_n == 2240) return launch_mx_dtype<240, 2>(a, lda, b, ldb, p, st);
+  // As long as all 128 x 128 tiles run at once they are the fastest: twice the SMs pull weights, and six stages of 32 KB
+  // keep more of them in flight.  us, 128 x 256 / 128 x 128 (tiles of the latter), the same bits: 16 x 10240 x 8192
+  // 37.0 / 24.9 (80), 128 x 8192 x 8192 38.0 / 24.4 (64), 512 x 4096 x 7168 33.2 / 22.3 (128), 1024 x 1280 x 8192
+  // 34.4 / 24.5 (80); in a second wave they lose: 256 x 10240 x 8192 41.2 / 47.5 (160).  (128 x 64 tiles gain 4 % more at
+  // 64-128 rows and lose up to 20 % below.)
+  if (((M + BM - 1) / BM) * ((N + 127) / 128) <= sm_count()) return launch_mx_dtype<128, 1>(a, lda, b, ldb, p, st);
   if (M >= 1024 && K >= 12288) return launch_mx_dtype<240, 2>(a, lda, b, ldb, p, st);
   if (M >= 512 && M < 4096 && N >= 4096) {
     // a cluster launch can be refused where a plain one is not (no pair of SMs free, a tool that does not support

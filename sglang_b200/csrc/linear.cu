@@ -83,7 +83,7 @@ LinearPlan plan_linear(Arena& a, int64_t M, int64_t N, int64_t K, int scale_mode
   p.q = a.take<uint8_t>(static_cast<size_t>(M) * K);
   p.s_ld = align4(M);
   p.s = a.take<uint32_t>(static_cast<size_t>(p.s_ld) * (ue8m0 ? (groups + 3) / 4 : groups));
-  p.partial_bytes = scale_mode != 2 || packed_promotes(M) ? b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) : 0;
+  p.partial_bytes = scale_mode != 2 || packed_promotes(M, N, K) ? b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K) : 0;
   p.partial = p.partial_bytes ? a.take<uint8_t>(p.partial_bytes) : nullptr;
   return p;
 }
@@ -121,7 +121,7 @@ extern "C" int b200_fp8_linear(const void* x, int dtype, const void* w, int64_t 
     rc = b200_per_token_group_quant_fp8_ue8m0(x, dtype, p.q, static_cast<uint32_t*>(p.s), M, K, p.s_ld, kQuantEps, -kFp8Max,
                                               kFp8Max, stream);
   if (rc != B200_OK) return rc;
-  if (scale_mode == 2 && !packed_promotes(M)) {
+  if (scale_mode == 2 && !packed_promotes(M, N, K)) {
     rc = b200_fp8_blockwise_scaled_mm_pow2(p.q, K, w, ldw, static_cast<uint32_t*>(p.s), 1, p.s_ld, ws, ws_stride_n,
                                            ws_stride_g, out, ldo, dtype, M, N, K, stream);
     return rc == B200_OK && bias ? bias_add(out, bias, M, N, ldo, dtype, st) : rc;
