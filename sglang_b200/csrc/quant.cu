@@ -403,13 +403,21 @@ __global__ void __launch_bounds__(kThreads, NV <= 2 ? (HAS_RES ? 4 : 5) : 2) rms
   [[maybe_unused]] Vec16<T> r[HAS_RES ? NV : 1];
   constexpr bool has_res = HAS_RES;
   float sumsq = 0.f;
+  // every load first: a store of the new residual between them would hold back the loads behind it (one DRAM round trip
+  // per 4096 columns; with the residual, before -> now: 2048 x 7168 21.8 -> 19.2 us, 16384 x 16384 419 -> 336 us)
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int v = tid + i * kThreads;
     if (v < nvec) {
       d[i].load(x + row * K + static_cast<int64_t>(v) * kVec);
+      if constexpr (HAS_RES) r[i].load(residual + row * K + static_cast<int64_t>(v) * kVec);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int v = tid + i * kThreads;
+    if (v < nvec) {
       if constexpr (HAS_RES) {
-        r[i].load(residual + row * K + static_cast<int64_t>(v) * kVec);
         float f[kVec];
 #pragma unroll
         for (int e = 0; e < kVec; ++e) {
@@ -483,9 +491,11 @@ int launch_group(const void* x, void* q, float* s, int64_t M, int64_t K, int64_t
   const int tiles_k = static_cast<int>((K + kTileW - 1) / kTileW);
   const int sms = sm_count();
   if (sms <= 0) return B200_ERR_CUDA;
-  // 4 passes (16 rows, 64 registers, 4 blocks per SM) measured fastest; 8 is kept for experiments
+  // 4 passes (16 rows, 64 registers, 4 blocks per SM) measured fastest; 8 is kept for experiments.  With the activation in
+  // front a pass needs gate and up at once: two passes (32768 x 2048: 84 us; four 89, one 89; it is bound by the exponential,
+  // the division and the conversions, some 45 instructions an element).
   constexpr int kMaxPasses = sizeof(T) == 4 ? 4 : 8;
-  constexpr int kDefaultPasses = 4;
+  constexpr int kDefaultPasses = FUSE_SILU ? 2 : 4;
   auto tiles_for = [&](int passes) { return ((M + 4 * passes - 1) / (4 * passes)) * tiles_k; };
   int passes = kDefaultPasses;
   while (passes > 1 && tiles_for(passes) < 4LL * sms) passes >>= 1;
