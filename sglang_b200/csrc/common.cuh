@@ -269,13 +269,6 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y,
-                                            int z) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
-      : "memory");
-}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
@@ -412,58 +405,11 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// One thread of the leader CTA issues; both SMs of the pair execute (M = 256 split 128 + 128).
-__device__ __forceinline__ void umma_f8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // Completion of the pair's MMAs arrives on the same-offset mbarrier in every CTA of `cta_mask`.
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t cta_mask) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
       ::"r"(smem_u32(bar)), "h"(cta_mask)
-      : "memory");
-}
-
-// One k-block of pair MMAs (four K=32 steps, fresh accumulator) plus its completion commit, issued
-// by the elected lane, bracketed by the barrier tests for the NEXT k-block: the two try_waits are
-// started first and their results are only read after the MMAs have been issued, so their latency
-// overlaps the issue instead of preceding it.  All lanes execute the tests (warp-uniform flow).
-__device__ __forceinline__ void umma_f8_pair_kblock_with_peek(
-    uint32_t elected, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint64_t* done_bar,
-    uint16_t cta_mask, uint64_t* next_acc_bar, uint32_t next_acc_parity, uint64_t* next_full_bar,
-    uint32_t next_full_parity, uint32_t& acc_ready, uint32_t& ops_ready) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred PE, PA, PF, PT, PZ;\n\t"
-      ".reg .b64 ad, bd;\n\t"
-      "setp.ne.b32 PE, %2, 0;\n\t"
-      "setp.eq.b32 PT, 0, 0;\n\t"
-      "setp.ne.b32 PZ, 0, 0;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 PA, [%9], %10;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 PF, [%11], %12;\n\t"
-      "@PE tcgen05.mma.cta_group::2.kind::f8f6f4 [%3], %4, %5, %6, PZ;\n\t"
-      "add.s64 ad, %4, 2;\n\t"
-      "add.s64 bd, %5, 2;\n\t"
-      "@PE tcgen05.mma.cta_group::2.kind::f8f6f4 [%3], ad, bd, %6, PT;\n\t"
-      "add.s64 ad, %4, 4;\n\t"
-      "add.s64 bd, %5, 4;\n\t"
-      "@PE tcgen05.mma.cta_group::2.kind::f8f6f4 [%3], ad, bd, %6, PT;\n\t"
-      "add.s64 ad, %4, 6;\n\t"
-      "add.s64 bd, %5, 6;\n\t"
-      "@PE tcgen05.mma.cta_group::2.kind::f8f6f4 [%3], ad, bd, %6, PT;\n\t"
-      "@PE tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%7], %8;\n\t"
-      "selp.b32 %0, 1, 0, PA;\n\t"
-      "selp.b32 %1, 1, 0, PF;\n\t"
-      "}\n"
-      : "=r"(acc_ready), "=r"(ops_ready)
-      : "r"(elected), "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(smem_u32(done_bar)), "h"(cta_mask),
-        "r"(smem_u32(next_acc_bar)), "r"(next_acc_parity), "r"(smem_u32(next_full_bar)), "r"(next_full_parity)
       : "memory");
 }
 

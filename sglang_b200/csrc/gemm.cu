@@ -80,10 +80,10 @@ __device__ __forceinline__ void tile_coords(int tile, int m_blocks, int n_blocks
 
 // Where a tile lives.  Dense: tiles of the [M, N] output, rasterised in groups of kGroupM row blocks.
 // Grouped: the row tiles of all experts laid end to end (tile_m_start[e] = first row tile of expert e,
-// in shared memory), n-blocks fastest so that neighbouring pairs stream different slices of the same
+// in shared memory), n-blocks fastest so that neighbouring CTAs stream different slices of the same
 // expert's weights while sharing its few activation rows through L2.
 struct TileInfo {
-  int row0;        // first row of A / out of the PAIR's tile
+  int row0;        // first row of A / out of the tile
   int valid_rows;  // rows of the tile that belong to the problem (<= TILE_M)
   int n0;          // first output column
   int b_row0;      // first row of the [E*N, K] weight matrix
@@ -126,7 +126,7 @@ __device__ __forceinline__ TileInfo get_tile(int tile, const GemmParams& p, int 
   return t;
 }
 
-// One unit of a pair's work list: a whole tile, or one split of a tile's k-blocks.
+// One unit of a CTA's work list: a whole tile, or one split of a tile's k-blocks.
 struct Work {
   int tile, split, kb_begin, kb_end;
   bool partial;   // the result is a partial sum for the workspace, not an output tile
@@ -204,7 +204,7 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   // ====================================================================== helper warpgroup
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kHelperRegs));
   if (warp == kTmaWarp) {
-    // ------------------------------------------------------------------ TMA producer (each CTA)
+    // ------------------------------------------------------------------ TMA producer
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -254,7 +254,7 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
     __syncwarp();
   } else if (warp == kMmaWarp) {
-    // ------------------------------------------------------------------ MMA issuer (leader CTA only)
+    // ------------------------------------------------------------------ MMA issuer
     // The whole warp walks the loop so that addresses and descriptors stay warp-uniform; one elected lane issues.
     const uint64_t a_desc0 = umma_desc_k128(smem_a);
     const uint64_t b_desc0 = umma_desc_k128(smem_b);
@@ -951,7 +951,7 @@ extern "C" int b200_fp8_blockwise_scaled_grouped_mm(const void* a, int64_t lda, 
     if (tt == 0) tt = avg_rows <= 20 ? 32 : 64;
     return launch_gemm_swapab(a, lda, total_rows, b, ldb, N * num_experts, p, true, tt, st);
   }
-  // 256-wide tiles unless they would leave pairs idle; a 128-column remainder (N % 256 != 0) costs its half only.
+  // 256-wide tiles unless they would leave half of the SMs idle; a 128-column remainder (N % 256 != 0) costs its half only.
   const int64_t tiles = (total_rows / TILE_M + num_experts) * ((N + 255) / 256);
   p.tile_n = g_force_block_n == 128 || (g_force_block_n != 256 && 2 * tiles < sm_count()) ? 128 : 256;
   CUtensorMap ma, mb;

@@ -24,15 +24,15 @@ struct GemmParams {
   int split_k;
   int kb_per_split;
   float* partial;
-  // tail split (dense, CTA-pair kernel): tiles [0, tail_first) are whole; each tile from tail_first on -- the ones
-  // that would form a mostly empty last wave -- is divided among split_k pairs.  partial_tiles != 0: partial sums are
-  // whole tiles, partial[(tile - tail_first) * split_k + split][256][tile_n]
+  // tail split (dense, 128-row-tile kernel): tiles [0, tail_first) are whole; each tile from tail_first on -- the ones
+  // that would form a mostly empty last wave -- is divided among split_k CTAs.  partial_tiles != 0: partial sums are
+  // whole tiles, partial[(tile - tail_first) * split_k + split][128][tile_n]
   int tail_first;
   int partial_tiles;
   const void* bias; // [N] in the output type, added to the rounded product; or nullptr
   int prefetch_w;   // != 0: the kernel before this one in the stream is this library's own and triggered after its wait, so
                     // weights may be fetched ahead of the wait
-  int tile_n;       // tile width of the CTA-pair kernel, 128 or 256
+  int tile_n;       // tile width of the 128-row-tile kernel, 128 or 256
   // activation scales given as packed UE8M0 exponent bytes (four k-blocks per 32-bit word) instead of fp32:
   // element (m, kb) is byte kb % 4 of the word at sa[(kb / 4) * sa_stride_g + m * sa_stride_m]
   int sa_ue8m0;
