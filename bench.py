@@ -1129,7 +1129,7 @@ def run_gpu_arm(args):
         launches_per_step = (1 + 1 + int(split1)) + chunks_used * (1 + 1 + int(split2)) + (chunks_used if ar is not None else 0)
         h2d = x_host.numel() * 2 + h.numel() * 2
         d2h = M_TOKENS * n1 * 2 + mr * HIDDEN * 2
-        roof = {"bound": "tensor", "kernel": "gemm_block_fp8_kernel<BLOCK_N=256, 16 epilogue warps, 32-column chunks, bf16> "
+        roof = {"bound": "tensor", "kernel": "gemm_block_fp8_kernel<BLOCK_N=256, 8 epilogue warps, 64-column chunks, bf16> "
                                              f"(gate_up{'' if world == 1 else f' shard N={n1}'})",
                 "achieved": achieved, "peak": peak_burst, "unit": "TFLOP/s", "frac": achieved / peak_burst,
                 "peak_source": f"2 x bf16_tflops (burst) of {pk['src']}: the kernel is timed with events inside a short eager pass "
