@@ -113,7 +113,7 @@ def deepgemm_w8a8_block_fp8_linear_with_fallback(input: torch.Tensor, weight: to
     power-of-two weight scales too (requant_weight_ue8m0): the product then runs on the tensor core's
     block-scaling path, all k-blocks accumulated in tensor memory."""
     assert input_scale is None
-    if scale_ue8m0 and list(block_size) == [128, 128]:
+    if gemm.SPLIT_K_MODE == "auto" and scale_ue8m0 and list(block_size) == [128, 128]:
         done = _lib.host().linear(input, weight, weight_scale, bias, None, 2 if weight_scale_ue8m0 else 1)
         if done is not None:
             return done

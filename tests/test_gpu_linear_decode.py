@@ -50,3 +50,22 @@ def test_decode_linear_power_of_two_scales(M, N):
     b_f = (w_f * ws.view(N // 128, 1, K // 128, 1)).reshape(N, K)
     exact = (a_f.double() @ b_f.double().T).to(torch.bfloat16)
     assert O.rel_l2(ref.float().cpu(), exact.float().cpu()) <= 1e-3
+
+
+@pytest.mark.parametrize("pow2_weights", [False, True])
+@pytest.mark.parametrize("M,N,K", [(16, 1280, 8192), (200, 640, 7168)])
+def test_power_of_two_linear_obeys_the_split_switch(M, N, K, pow2_weights, monkeypatch):
+    """Sizes that the automatic mode splits: with the switch off, the bits of the unsplit product."""
+    from sglang_b200.layers.quantization.fp8_kernel import sglang_per_token_group_quant_fp8, w8a8_block_fp8_matmul_deepgemm
+    from sglang_b200.layers.quantization.fp8_utils import (deepgemm_w8a8_block_fp8_linear_with_fallback,
+                                                            requant_weight_ue8m0)
+    from sglang_b200.sgl_kernel import gemm
+    x = torch.randn(M, K, generator=torch.Generator(device="cuda").manual_seed(M), device="cuda").to(torch.bfloat16)
+    wq, ws = O.gen_weight(N, K, seed=N)
+    wq, ws = requant_weight_ue8m0(wq.cuda(), ws.cuda(), [128, 128])
+    q, s = sglang_per_token_group_quant_fp8(x, 128, column_major_scales=True, scale_tma_aligned=True, scale_ue8m0=True)
+    unsplit = w8a8_block_fp8_matmul_deepgemm(q, wq, s, ws, [128, 128], torch.bfloat16, weight_scale_ue8m0=pow2_weights)
+    assert gemm._splitk_plan(M, N, K, x.device)[0] > 1, "the sizes are meant to be split"
+    monkeypatch.setattr(gemm, "SPLIT_K_MODE", "off")
+    out = deepgemm_w8a8_block_fp8_linear_with_fallback(x, wq, [128, 128], ws, weight_scale_ue8m0=pow2_weights)
+    assert torch.equal(out, unsplit)
