@@ -186,23 +186,23 @@ int b200_fp8_blockwise_scaled_mm(const void* a, int64_t lda, const void* b, int6
                                  int64_t M, int64_t N, int64_t K, void* stream);
 
 /*
- * The same product for small M (M <= 512), with the k-blocks of each output tile divided among
- * `split_k` CTAs so that the weight matrix streams through every SM even when the output has only a
- * few tiles (decode-size batches of the DeepSeek-V3 down projection: 28 tiles on 148 SMs).  Each CTA
- * writes fp32 partial sums to workspace[split][M][N]; a second kernel adds them in split order and
- * converts, so results are deterministic.  The fp32 sum over k-blocks is grouped differently from the
- * unsplit kernel, so the two agree to rounding (same parity tolerance), not bit for bit.
- *   split_k  0 = chosen by the library (falls back to 1 when the workspace is missing or too small);
- *            1 = identical to b200_fp8_blockwise_scaled_mm; 2..64 = forced (needs N % 4 == 0,
- *            split_k <= ceil(K/128))
- *   workspace  device memory, 16-byte aligned, at least split_k * M * N * 4 bytes; never allocated here
- * With split_k = 0 and M > 128 the library may instead split only the LAST WAVE of output tiles: when
- * tiles mod SMs is at most half of the SMs (896 tiles on 148 SMs leave a seventh wave of 8 tiles),
- * those tiles' k-blocks are divided among the SMs, their fp32 partial tiles go to the workspace (compact:
- * tail tiles x splits x 128 x tile width x 4 bytes) and a small second kernel adds them in split order.
- * Same rounding remark as above; the other tiles are bit-identical to the unsplit kernel.
- * b200_fp8_blockwise_scaled_mm_splitk_plan reports the split the library would choose for a shape on
- * a GPU with `sm_count` SMs (<= 0: 148) and the workspace that needs; it touches no device.
+ * The same product with the k-blocks of output tiles divided among several CTAs, so that the weight matrix streams
+ * through every SM even when the output has few tiles (decode-size batches of the DeepSeek-V3 down projection: 56 tiles
+ * on 148 SMs).  Each CTA writes fp32 partial sums to the workspace; a second kernel adds them in split order and
+ * converts, so results are deterministic.  The fp32 sum over k-blocks is grouped differently from the unsplit kernel,
+ * so the two agree to rounding (same parity tolerance), not bit for bit.
+ *   split_k  0 = the library's own schedule, as far as the workspace allows (none or too little: it splits less or not
+ *            at all); 1 = identical to b200_fp8_blockwise_scaled_mm; 2..64 = every tile is divided in that many (needs
+ *            N % 4 == 0, split_k <= ceil(K/128))
+ *   workspace  device memory, 16-byte aligned; for split_k >= 2 at least split_k * M * N * 4 bytes, for split_k = 0 what
+ *            the plan or b200_fp8_blockwise_scaled_mm_workspace_bytes says; never allocated here
+ * The library's own schedule: few tokens (up to 64, and up to 192 where its tiles fit into a wave) run on the
+ * weight-streaming kernel, all of whose tiles are divided when they would leave SMs idle.  Otherwise only the LAST WAVE
+ * of 128 x 256 or 128 x 128 tiles is (which is all of them when there are fewer tiles than SMs), where a model of the
+ * longest CTA's cycles says that it pays; the other tiles are bit-identical to the unsplit kernel.
+ * b200_fp8_blockwise_scaled_mm_splitk_plan reports that schedule for a GPU with `sm_count` SMs (b200_sm_count() for the
+ * current device; <= 0: 148): into how many CTAs' k-blocks a divided tile goes (1: none is divided) and the workspace
+ * that split_k = 0 uses for it.  It touches no device.
  * No counterpart in the reference (its CUTLASS kernel has no split-K form; the Triton kernel at
  * python/sglang/srt/layers/quantization/fp8_kernel.py:849-966 covers small M with smaller tiles).
  */
@@ -441,15 +441,16 @@ int b200_topk_softmax(const void* gating_output, int dtype, int64_t row_stride, 
  * `dtype` (bf16 / fp16); bias is added to the rounded product.  K % 128 == 0.
  * scale_mode 0: fp32 scales; 1: power-of-two activation scales; 2: weight scales are powers of two as well.
  * Everything in between lives in `workspace` (b200_fp8_linear_workspace_bytes bytes, 16-byte aligned), which may be
- * reused by the next call on the same stream.  b200_sm_count: SMs the persistent kernels use on the current device.
+ * reused by the next call on the same stream.  b200_sm_count: SMs the persistent kernels use on the current device
+ * (its SMs, or the limit of b200_set_sm_limit).
  */
 size_t b200_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K, int scale_mode);
 int b200_fp8_linear(const void* x, int dtype, const void* w, int64_t ldw, const float* ws, int64_t ws_stride_n,
                     int64_t ws_stride_g, const void* bias, void* out, int64_t ldo, int64_t M, int64_t N, int64_t K,
                     int scale_mode, void* workspace, size_t workspace_bytes, void* stream);
 int b200_sm_count(void);
-/* Workspace with which b200_fp8_blockwise_scaled_mm_splitk (split_k = 0) runs its best schedule on the current device;
- * with less it splits less. */
+/* Workspace with which b200_fp8_blockwise_scaled_mm_splitk (split_k = 0) runs its best schedule on the current device
+ * (the plan's figure for b200_sm_count() SMs); with less it splits less. */
 size_t b200_fp8_blockwise_scaled_mm_workspace_bytes(int64_t M, int64_t N, int64_t K);
 
 /*

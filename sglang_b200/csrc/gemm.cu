@@ -641,23 +641,18 @@ inline bool dense_uses_swapab(int64_t M, int64_t N, int sms) {
   return tiles <= sms || (M > 128 && 2 * tiles > 3 * sms && tiles <= 2 * sms);
 }
 
-// Split count for small M (up to 512 rows): when the output has too few tiles for the SMs, the k-blocks of
-// each tile are spread over several CTAs so that the weights stream through all SMs at once.
+// Split count of the weight-streaming kernel: when the output has too few tiles for the SMs, the k-blocks of each tile are
+// spread over several CTAs so that the weights stream through all SMs at once.
 int plan_split_k(int64_t M, int64_t N, int64_t K, int sms) {
-  if (M > 4 * TILE_M || (N % 4) != 0) return 1;   // beyond 512 rows the tile count is never that small
-  const int64_t m_blocks = (M + TILE_M - 1) / TILE_M;
+  if ((N % 4) != 0) return 1;
   const int64_t tt = dense_token_tile(M);
-  const bool stream = M <= kStreamTokens;
-  const int64_t tiles = stream ? ((M + tt - 1) / tt) * ((N + 127) / 128) : m_blocks * ((N + 255) / 256);
+  const int64_t tiles = ((M + tt - 1) / tt) * ((N + 127) / 128);
   const int64_t nkb = (K + BLOCK_K - 1) / BLOCK_K;
   // measured on DeepSeek-V3 shapes: below 32 k-blocks the launch and pipeline ramp dominate and the
   // extra reduce kernel costs more than the idle SMs
   if (nkb < 32) return 1;
   if (tiles * 2 > sms) {
-    // More tiles than half the SMs.  The weight-streaming kernel with two or three token tiles per weight tile can
-    // still leave most of its last wave empty (DeepSeek-V3 down projection at 129-192 tokens: 168 tiles on 148 SMs;
-    // measured 63.9 us unsplit, 55.5 us split in two): split only to fill such a wave.
-    if (!stream) return 1;
+    // More tiles than half the SMs: split only to fill a last wave that is mostly empty.
     auto fill = [sms](int64_t t) { return static_cast<double>(t) / static_cast<double>(((t + sms - 1) / sms) * sms); };
     if (fill(tiles) >= 0.7) return 1;
     for (int s2 = 2; s2 <= 4; ++s2)
@@ -678,29 +673,6 @@ int plan_split_k(int64_t M, int64_t N, int64_t K, int sms) {
 // the device-wide fences and the CTA-wide meeting it needs cost more than a launch.)
 inline size_t splitk_workspace_bytes(int split_k, int64_t M, int64_t N) {
   return static_cast<size_t>(split_k) * M * N * sizeof(float);
-}
-
-// Tail of the 128 x 256 tiling that b200_fp8_blockwise_scaled_mm_splitk_plan has always described: the workspace that
-// such a split takes, which is also a workspace the schedules below can use.
-struct TailPlan {
-  int split_k = 1;
-  size_t bytes = 0;
-};
-TailPlan plan_tail(int64_t M, int64_t N, int64_t K, int sms) {
-  TailPlan t;
-  const int64_t m_blocks = (M + 127) / 128;
-  const int block_n = 4 * m_blocks * ((N + 255) / 256) < 3 * sms ? 128 : 256;
-  const int64_t tiles = m_blocks * ((N + block_n - 1) / block_n);
-  const int64_t nkb = (K + BLOCK_K - 1) / BLOCK_K;
-  if (M <= 128 || tiles <= sms || tiles > 0x3fffffff || nkb < 16) return t;
-  const int64_t tail = tiles % sms;
-  if (tail == 0 || tail * 2 > sms) return t;   // at least two splits per tail tile
-  int64_t s = std::min<int64_t>({sms / tail, nkb / 4, 32});   // at least four k-blocks per work unit
-  if (s < 2) return t;
-  const int64_t kbps = (nkb + s - 1) / s;
-  t.split_k = static_cast<int>((nkb + kbps - 1) / kbps);
-  t.bytes = static_cast<size_t>(tail) * t.split_k * 128 * block_n * sizeof(float);
-  return t;
 }
 
 // Schedule of this file's kernel for a dense problem: tile width, and how many of the last tiles have their k-blocks
@@ -742,6 +714,32 @@ TilePlan plan_tiles(int64_t M, int64_t N, int64_t K, int sms, size_t max_bytes) 
     }
   }
   return best;
+}
+
+// What a dense problem runs with a workspace of up to max_bytes: the one answer behind dense_mm, the plan and the
+// workspace entry points.  bytes = workspace the schedule uses, 0 when nothing is split.
+struct DensePlan {
+  bool swapab = false;
+  int split_k = 1;        // CTAs per divided tile, either kernel
+  size_t bytes = 0;
+  TilePlan tiles;         // this file's kernel
+};
+DensePlan plan_dense(int64_t M, int64_t N, int64_t K, int sms, bool swapab, size_t max_bytes) {
+  DensePlan d;
+  d.swapab = swapab;
+  if (swapab) {
+    const int s = plan_split_k(M, N, K, sms);
+    const size_t bytes = s > 1 ? splitk_workspace_bytes(s, M, N) : 0;
+    if (bytes <= max_bytes) {
+      d.split_k = s;
+      d.bytes = bytes;
+    }
+  } else {
+    d.tiles = plan_tiles(M, N, K, sms, max_bytes);
+    d.split_k = d.tiles.split_k;
+    d.bytes = d.tiles.bytes;
+  }
+  return d;
 }
 
 }  // namespace
@@ -786,17 +784,12 @@ int dense_mm(const void* a, int64_t lda, const void* b, int64_t ldb, const float
   if (gemm_sticky_status() != 0) return B200_ERR_DEVICE_TIMEOUT;   // sticky until b200_gemm_device_status clears it
   TilePlan plan;
   const bool swapab = g_force_block_n == 3 || forced_token_tile() != 0 || (g_force_block_n == 0 && dense_uses_swapab(M, N, sm_count()));
-  if (!swapab && (split_k == 1 || (split_k == 0 && (!workspace || !aligned16(workspace)))))
-    plan = plan_tiles(M, N, K, sm_count(), 0);
-  if (split_k == 0) {
-    // automatic: split only when the caller gave room for it
-    split_k = 1;
-    if (swapab) {
-      const int s = plan_split_k(M, N, K, sm_count());
-      if (s > 1 && workspace && aligned16(workspace) && workspace_bytes >= splitk_workspace_bytes(s, M, N)) split_k = s;
-    } else if (workspace && aligned16(workspace)) {
-      plan = plan_tiles(M, N, K, sm_count(), workspace_bytes);
-    }
+  if (split_k <= 1) {
+    // automatic (0): split only when the caller gave room for it
+    const size_t room = split_k == 0 && workspace && aligned16(workspace) ? workspace_bytes : 0;
+    const DensePlan d = plan_dense(M, N, K, sm_count(), swapab, room);
+    plan = d.tiles;
+    split_k = swapab ? d.split_k : 1;
   }
   if (g_force_block_n == 128 || g_force_block_n == 256) {
     plan = TilePlan();
@@ -886,16 +879,12 @@ extern "C" int b200_fp8_blockwise_scaled_mm_splitk_plan(int64_t M, int64_t N, in
   if (M < 0 || N < 0 || K <= 0) return B200_ERR_BAD_SHAPE;
   if (!split_k || !workspace_bytes) return B200_ERR_NULL_PTR;
   const int sms = sm_count > 0 ? sm_count : 148;
-  const int s = (M == 0 || N == 0) ? 1 : b200::plan_split_k(M, N, K, sms);
-  *split_k = s;
-  *workspace_bytes = s > 1 ? b200::splitk_workspace_bytes(s, M, N) : 0;
-  if (s == 1 && M > 128 && M > b200::kStreamTokens && N > 0) {   // large M: split of the last, mostly empty wave of tiles
-    const b200::TailPlan t = b200::plan_tail(M, N, K, sms);
-    if (t.split_k > 1) {
-      *split_k = t.split_k;
-      *workspace_bytes = t.bytes;
-    }
-  }
+  *split_k = 1;
+  *workspace_bytes = 0;
+  if (M == 0 || N == 0) return B200_OK;
+  const b200::DensePlan d = b200::plan_dense(M, N, K, sms, b200::dense_uses_swapab(M, N, sms), ~size_t(0));
+  *split_k = d.split_k;
+  *workspace_bytes = d.bytes;
   return B200_OK;
 }
 
@@ -970,9 +959,5 @@ extern "C" int b200_debug_force_block_n(int block_n) {
 extern "C" size_t b200_fp8_blockwise_scaled_mm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (dense_uses_swapab(M, N, sm_count())) {
-    const int s = plan_split_k(M, N, K, sm_count());
-    return s > 1 ? splitk_workspace_bytes(s, M, N) : 0;
-  }
-  return plan_tiles(M, N, K, sm_count(), ~size_t(0)).bytes;
+  return plan_dense(M, N, K, sm_count(), dense_uses_swapab(M, N, sm_count()), ~size_t(0)).bytes;
 }

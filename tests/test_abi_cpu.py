@@ -80,34 +80,34 @@ def test_argument_checks_return_before_any_device_work(lib):
 
 
 def test_split_k_plan_needs_no_device(lib):
-    """Decode-size batches on narrow, deep projections split; wide or shallow ones do not."""
+    """The schedule that split_k = 0 runs: decode-size batches on narrow, deep projections split, wide or shallow ones do
+    not; the 128-row-tile kernel splits its last wave of tiles."""
     def plan(M, N, K, sms=148):
         s, b = ctypes.c_int(-1), ctypes.c_size_t(1)
         assert lib.b200_fp8_blockwise_scaled_mm_splitk_plan(M, N, K, sms, ctypes.byref(s), ctypes.byref(b)) == 0
-        if M <= 512:
-            assert b.value == (s.value * M * N * 4 if s.value > 1 else 0)
-        return s.value
-    assert plan(16, 7168, 18432) == 2          # <= 64 tokens: 56 tiles of 128 weight rows on 148 SMs
-    assert plan(128, 7168, 18432) == 1         # 65..128 tokens: two token tiles x 56 weight tiles, 76 % of one wave
-    assert plan(1, 1536, 7168) == 7            # capped at eight k-blocks per CTA
-    assert plan(16, 36864, 7168) == 1          # already more tiles than SMs
-    assert plan(16, 7168, 2048) == 1           # too few k-blocks to pay for the reduce kernel
-    assert plan(129, 7168, 18432) == 2         # three token tiles x 56: 168 tiles, a nearly empty second wave
-    assert plan(192, 10240, 8192) == 1         # 240 tiles: 81 % of two waves
-    assert plan(256, 7168, 18432) == 2         # beyond 192 tokens 128 x 256 tiles: 56 of them
-    assert plan(512, 7168, 18432) == 1         # 112 tiles: most SMs busy already
-    assert plan(0, 7168, 18432) == 1
-    assert plan(16, 7168, 18432, sms=0) == 2   # <= 0 means a 148-SM part
+        assert (s.value > 1) == (b.value > 0)
+        return s.value, b.value
+    # weight-streaming kernel: planes of the whole output
+    assert plan(16, 7168, 18432) == (2, 2 * 16 * 7168 * 4)      # <= 64 tokens: 56 tiles of 128 weight rows on 148 SMs
+    assert plan(128, 7168, 18432) == (1, 0)    # 65..128 tokens: two token tiles x 56 weight tiles, 76 % of one wave
+    assert plan(1, 1536, 7168) == (7, 7 * 1536 * 4)             # capped at eight k-blocks per CTA
+    assert plan(16, 36864, 7168) == (1, 0)     # already more tiles than SMs
+    assert plan(16, 7168, 2048) == (1, 0)      # too few k-blocks to pay for the reduce kernel
+    assert plan(192, 10240, 8192) == (1, 0)    # 240 tiles: 81 % of two waves
+    # 128-row tiles, fewer of them than SMs: planes of whole tiles
+    assert plan(129, 7168, 18432) == (2, 56 * 2 * 128 * 256 * 4)
+    assert plan(256, 7168, 18432) == (2, 56 * 2 * 128 * 256 * 4)
+    assert plan(1021, 576, 7168) == (3, 40 * 3 * 128 * 128 * 4)     # 128-wide tiles: twice as many of them
+    assert plan(512, 7168, 18432) == (1, 0)    # 112 tiles: most SMs busy already
+    assert plan(0, 7168, 18432) == (1, 0)
+    assert plan(16, 7168, 18432, sms=0) == plan(16, 7168, 18432)    # <= 0 means a 148-SM part
     # large M: only the last, mostly empty wave of tiles is split
-    assert plan(4096, 7168, 18432) == 18       # 896 tiles of 128 x 256: six waves + 8 tiles -> 8 x 18 work units
-    s, b = ctypes.c_int(0), ctypes.c_size_t(0)
-    assert lib.b200_fp8_blockwise_scaled_mm_splitk_plan(4096, 7168, 18432, 148, ctypes.byref(s), ctypes.byref(b)) == 0
-    assert b.value == 8 * 18 * 128 * 256 * 4
-    assert plan(4096, 36864, 7168) == 7        # 4608 tiles: 31 waves + 20 tiles
-    assert plan(16384, 36864, 7168) == 1       # 18432 tiles: the last wave is 80 tiles, more than half of the SMs
-    assert plan(8192, 2560, 8192) == 3         # 640 tiles: four waves + 48 tiles -> 48 x 3 work units
-    assert plan(8192, 1280, 8192) == 6         # 320 tiles: two waves + 24 tiles
-    assert plan(4096, 7168, 1024) == 1         # too few k-blocks to divide
+    assert plan(4096, 7168, 18432) == (9, 8 * 9 * 128 * 256 * 4)      # 896 tiles of 128 x 256: six waves + 8 tiles
+    assert plan(4096, 36864, 7168) == (4, 20 * 4 * 128 * 256 * 4)     # 4608 tiles: 31 waves + 20 tiles
+    assert plan(16384, 36864, 7168) == (1, 0)  # 18432 tiles: the last wave is 80 tiles, more than half of the SMs
+    assert plan(8192, 2560, 8192) == (3, 48 * 3 * 128 * 256 * 4)      # 640 tiles: four waves + 48 tiles
+    assert plan(8192, 1280, 8192) == (4, 24 * 4 * 128 * 256 * 4)      # 320 tiles: two waves + 24 tiles
+    assert plan(4096, 7168, 1024) == (1, 0)    # too few k-blocks to divide
     s, b = ctypes.c_int(0), ctypes.c_size_t(0)
     assert lib.b200_fp8_blockwise_scaled_mm_splitk_plan(-1, 128, 128, 148, ctypes.byref(s), ctypes.byref(b)) < 0
     assert lib.b200_fp8_blockwise_scaled_mm_splitk_plan(1, 128, 128, 148, None, None) < 0

@@ -34,3 +34,32 @@ def test_linear_bias_is_added_to_the_rounded_product(M, dtype):
     with_bias = w8a8_block_fp8_linear(x, wq.cuda(), [128, 128], ws.cuda(), bias=bias)
     plain += bias
     assert torch.equal(plain, with_bias)
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 7168, 8192), (129, 7168, 8192), (1021, 576, 7168), (1300, 4040, 5248), (64, 128, 128)])
+def test_plan_is_what_the_library_runs(M, N, K):
+    """The plan's workspace is the one that the automatic schedule uses: the workspace entry point gives the same figure,
+    with it the result has the bits of the torch-facing call, and nothing is written beyond it."""
+    import ctypes
+    from sglang_b200 import _lib
+    from sglang_b200.layers.quantization.fp8_kernel import w8a8_block_fp8_matmul
+    L = _lib.lib()
+    split, nbytes = ctypes.c_int(0), ctypes.c_size_t(0)
+    _lib.check("plan", L.b200_fp8_blockwise_scaled_mm_splitk_plan(M, N, K, L.b200_sm_count(), ctypes.byref(split), ctypes.byref(nbytes)))
+    assert nbytes.value == L.b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K)
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = (torch.randn(M, K, generator=g, device="cuda") * 60).clamp(-448, 448).to(torch.float8_e4m3fn)
+    b = (torch.randn(N, K, generator=g, device="cuda") * 60).clamp(-448, 448).to(torch.float8_e4m3fn)
+    sa = torch.rand(M, K // 128, generator=g, device="cuda") * 0.01
+    sb = torch.rand((N + 127) // 128, K // 128, generator=g, device="cuda") * 0.01
+    out = torch.empty(M, N, device="cuda")
+    n = nbytes.value // 4
+    ws = torch.full((n + 1024,), 123.0, device="cuda")
+    _lib.check("mm", L.b200_fp8_blockwise_scaled_mm_splitk(
+        a.data_ptr(), K, b.data_ptr(), K, sa.data_ptr(), K // 128, 1, sb.data_ptr(), K // 128, 1, out.data_ptr(), N,
+        _lib.DT_F32, M, N, K, 0, ws.data_ptr() if n else None, nbytes.value, torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert torch.equal(out, w8a8_block_fp8_matmul(a, b, sa, sb, [128, 128], torch.float32))
+    assert bool((ws[n:] == 123.0).all())
+    used = int((ws[:n] != 123.0).sum())
+    assert (used > 0) == (split.value > 1)
