@@ -18,6 +18,8 @@
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <vector>
+
 #include "../../include/b200_block_fp8.h"
 
 namespace {
@@ -58,6 +60,17 @@ void* stream_of(const at::Device& dev) { return c10::cuda::getCurrentCUDAStream(
 
 PyObject* none() { Py_RETURN_NONE; }
 
+// The interpreter lock is free while this lives.  Allocating may wait for the device and a launch for room in the queue;
+// the process's other Python threads go on meanwhile, as they do under a ctypes call.  Everything that is read from a
+// Python-owned tensor is read before; tensors held by value are fine.
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  NoGil() = default;
+  NoGil(const NoGil&) = delete;
+  NoGil& operator=(const NoGil&) = delete;
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 // Raises _lib.B200Error(fn, code, detail), the exception the Python functions raise.
 PyObject* raise_status(const char* fn, int code) {
   PyObject* mod = PyImport_ImportModule("sglang_b200._lib");
@@ -72,9 +85,10 @@ PyObject* raise_status(const char* fn, int code) {
 
 int64_t align4(int64_t v) { return (v + 3) / 4 * 4; }
 
-// Scale tensor of sglang_per_token_group_quant_fp8 for x [..., K] seen as [M, K]; `rs` and `gs` are its strides.
+// Scale tensor of sglang_per_token_group_quant_fp8 for x [..., K] of these sizes seen as [M, K]; `rs` and `gs` are its
+// strides.
 // Packed words are zero-filled where the quantiser may leave bytes alone (`partial`) or rows are padding.
-Tensor scale_tensor(const Tensor& x, int64_t K, int64_t M, int64_t group, bool col_major, bool aligned, bool ue8m0,
+Tensor scale_tensor(std::vector<int64_t> sizes, int64_t K, int64_t M, int64_t group, bool col_major, bool aligned, bool ue8m0,
                     bool partial, const at::Device& dev, int64_t& rs, int64_t& gs) {
   const int64_t G = K / group;
   if (ue8m0) {
@@ -95,7 +109,6 @@ Tensor scale_tensor(const Tensor& x, int64_t K, int64_t M, int64_t group, bool c
   }
   rs = G;
   gs = 1;
-  auto sizes = x.sizes().vec();
   sizes.back() = G;
   return empty(sizes, at::kFloat, dev);
 }
@@ -138,27 +151,32 @@ HOST_FN(linear) {
       return none();
   }
   const at::Device dev = x->device();
-  const c10::cuda::OptionalCUDAGuard guard(dev);
+  const at::ScalarType xt = x->scalar_type();
   Tensor out;
   int64_t ldo = N;
   auto out_sizes = x->sizes().vec();
   out_sizes.back() = N;
   if (a[4] != Py_None) {
-    const Tensor* o = cuda_tensor(a[4], x->scalar_type());
+    const Tensor* o = cuda_tensor(a[4], xt);
     if (!o || o->dim() != 2 || o->size(0) != M || o->size(1) != N || o->stride(1) != 1 || o->stride(0) < N ||
         o->device() != dev || x->dim() != 2)
       return none();
     ldo = o->stride(0);
     out = *o;
-  } else {
-    out = empty(out_sizes, x->scalar_type(), dev);
   }
-  const size_t bytes = b200_fp8_linear_workspace_bytes(M, N, K, static_cast<int>(mode));
-  const Tensor work = empty({static_cast<int64_t>(bytes)}, at::kByte, dev);
-  const int rc = b200_fp8_linear(x->data_ptr(), dt_of(x->scalar_type()), w->data_ptr(), K,
-                                 static_cast<const float*>(ws->data_ptr()), ws->stride(0), ws->stride(1),
-                                 bias ? bias->data_ptr() : nullptr, out.data_ptr(), ldo, M, N, K, static_cast<int>(mode),
-                                 work.data_ptr(), bytes, stream_of(dev));
+  const void *xp = x->data_ptr(), *wp = w->data_ptr(), *bp = bias ? bias->data_ptr() : nullptr;
+  const float* wsp = static_cast<const float*>(ws->data_ptr());
+  const int64_t ws_n = ws->stride(0), ws_g = ws->stride(1);
+  int rc;
+  {
+    const NoGil no_gil;
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    if (!out.defined()) out = empty(out_sizes, xt, dev);
+    const size_t bytes = b200_fp8_linear_workspace_bytes(M, N, K, static_cast<int>(mode));
+    const Tensor work = empty({static_cast<int64_t>(bytes)}, at::kByte, dev);
+    rc = b200_fp8_linear(xp, dt_of(xt), wp, K, wsp, ws_n, ws_g, bp, out.data_ptr(), ldo, M, N, K, static_cast<int>(mode),
+                         work.data_ptr(), bytes, stream_of(dev));
+  }
   if (rc != 0) return raise_status("fp8_linear", rc);
   return THPVariable_Wrap(std::move(out));
 }
@@ -178,17 +196,23 @@ HOST_FN(quant) {
   if ((col || ue8m0) && x->dim() != 2) return none();
   if (ue8m0 && !(col && aligned && group == 128)) return none();
   const at::Device dev = x->device();
-  const c10::cuda::OptionalCUDAGuard guard(dev);
   const int64_t M = x->numel() / K;
-  Tensor q = empty(x->sizes(), at::kFloat8_e4m3fn, dev);
-  int64_t rs, gs;
-  Tensor s = scale_tensor(*x, K, M, group, col, aligned, ue8m0, false, dev, rs, gs);
-  void* st = stream_of(dev);
-  const int rc = ue8m0 ? b200_per_token_group_quant_fp8_ue8m0(x->data_ptr(), dt, q.data_ptr(),
-                                                              static_cast<uint32_t*>(s.data_ptr()), M, K, gs,
-                                                              static_cast<float>(eps), -448.0f, 448.0f, st)
-                       : b200_per_token_group_quant_fp8(x->data_ptr(), dt, q.data_ptr(), static_cast<float*>(s.data_ptr()),
-                                                        M, K, group, rs, gs, static_cast<float>(eps), -448.0f, 448.0f, st);
+  const auto sizes = x->sizes().vec();
+  const void* xp = x->data_ptr();
+  Tensor q, s;
+  int rc;
+  {
+    const NoGil no_gil;
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    q = empty(sizes, at::kFloat8_e4m3fn, dev);
+    int64_t rs, gs;
+    s = scale_tensor(sizes, K, M, group, col, aligned, ue8m0, false, dev, rs, gs);
+    void* st = stream_of(dev);
+    rc = ue8m0 ? b200_per_token_group_quant_fp8_ue8m0(xp, dt, q.data_ptr(), static_cast<uint32_t*>(s.data_ptr()), M, K, gs,
+                                                      static_cast<float>(eps), -448.0f, 448.0f, st)
+               : b200_per_token_group_quant_fp8(xp, dt, q.data_ptr(), static_cast<float*>(s.data_ptr()), M, K, group, rs, gs,
+                                                static_cast<float>(eps), -448.0f, 448.0f, st);
+  }
   if (rc != 0) return raise_status("sgl_per_token_group_quant_fp8", rc);
   return pair_of(std::move(q), std::move(s));
 }
@@ -212,14 +236,22 @@ HOST_FN(norm_quant) {
   if (PyErr_Occurred()) return nullptr;
   if (x->dim() != 2 || (ue8m0 && !(col && aligned)) || w->device() != x->device()) return none();
   const at::Device dev = x->device();
-  const c10::cuda::OptionalCUDAGuard guard(dev);
-  Tensor q = empty(x->sizes(), at::kFloat8_e4m3fn, dev);
-  int64_t rs, gs;
-  Tensor s = scale_tensor(*x, K, M, 128, col, aligned, ue8m0, true, dev, rs, gs);
-  const int rc = b200_rmsnorm_per_token_group_quant_fp8(
-      x->data_ptr(), dt_of(x->scalar_type()), r ? r->data_ptr() : nullptr, w->data_ptr(), static_cast<float>(norm_eps),
-      nullptr, q.data_ptr(), s.data_ptr(), M, K, rs, gs, ue8m0 ? 1 : 0, static_cast<float>(eps), -448.0f, 448.0f,
-      stream_of(dev));
+  const auto sizes = x->sizes().vec();
+  const int dt = dt_of(x->scalar_type());
+  const void *xp = x->data_ptr(), *wp = w->data_ptr();
+  void* rp = r ? r->data_ptr() : nullptr;
+  Tensor q, s;
+  int rc;
+  {
+    const NoGil no_gil;
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    q = empty(sizes, at::kFloat8_e4m3fn, dev);
+    int64_t rs, gs;
+    s = scale_tensor(sizes, K, M, 128, col, aligned, ue8m0, true, dev, rs, gs);
+    rc = b200_rmsnorm_per_token_group_quant_fp8(xp, dt, rp, wp, static_cast<float>(norm_eps), nullptr, q.data_ptr(),
+                                                s.data_ptr(), M, K, rs, gs, ue8m0 ? 1 : 0, static_cast<float>(eps), -448.0f,
+                                                448.0f, stream_of(dev));
+  }
   if (rc != 0) return raise_status("rmsnorm_per_token_group_quant_fp8", rc);
   return pair_of(std::move(q), std::move(s));
 }
@@ -233,11 +265,19 @@ HOST_FN(silu_and_mul) {
   const int64_t d2 = x->size(-1), d = d2 / 2;
   if (d2 % 16 != 0) return none();
   const at::Device dev = x->device();
-  const c10::cuda::OptionalCUDAGuard guard(dev);
+  const at::ScalarType xt = x->scalar_type();
   auto sizes = x->sizes().vec();
   sizes.back() = d;
-  Tensor out = empty(sizes, x->scalar_type(), dev);
-  const int rc = b200_silu_and_mul(x->data_ptr(), out.data_ptr(), x->numel() / d2, d, dt_of(x->scalar_type()), stream_of(dev));
+  const int64_t rows = x->numel() / d2;
+  const void* xp = x->data_ptr();
+  Tensor out;
+  int rc;
+  {
+    const NoGil no_gil;
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    out = empty(sizes, xt, dev);
+    rc = b200_silu_and_mul(xp, out.data_ptr(), rows, d, dt_of(xt), stream_of(dev));
+  }
   if (rc != 0) return raise_status("silu_and_mul", rc);
   return THPVariable_Wrap(std::move(out));
 }
@@ -257,15 +297,21 @@ HOST_FN(matmul) {
   if (xs->size(0) != M || xs->size(1) != K / 128 || ws->size(0) != (N + 127) / 128 || ws->size(1) != K / 128) return none();
   const at::Device dev = x->device();
   if (w->device() != dev || xs->device() != dev || ws->device() != dev) return none();
-  const c10::cuda::OptionalCUDAGuard guard(dev);
-  Tensor out = empty({M, N}, ot, dev);
-  const size_t bytes = b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K);
-  Tensor work;
-  if (bytes) work = empty({static_cast<int64_t>(bytes)}, at::kByte, dev);
-  const int rc = b200_fp8_blockwise_scaled_mm_splitk(
-      x->data_ptr(), K, w->data_ptr(), K, static_cast<const float*>(xs->data_ptr()), xs->stride(0), xs->stride(1),
-      static_cast<const float*>(ws->data_ptr()), ws->stride(0), ws->stride(1), out.data_ptr(), N, dt_of(ot), M, N, K, 0,
-      bytes ? work.data_ptr() : nullptr, bytes, stream_of(dev));
+  const void *xp = x->data_ptr(), *wp = w->data_ptr();
+  const float *xsp = static_cast<const float*>(xs->data_ptr()), *wsp = static_cast<const float*>(ws->data_ptr());
+  const int64_t xs_m = xs->stride(0), xs_g = xs->stride(1), ws_n = ws->stride(0), ws_g = ws->stride(1);
+  Tensor out;
+  int rc;
+  {
+    const NoGil no_gil;
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    out = empty({M, N}, ot, dev);
+    const size_t bytes = b200_fp8_blockwise_scaled_mm_workspace_bytes(M, N, K);
+    Tensor work;
+    if (bytes) work = empty({static_cast<int64_t>(bytes)}, at::kByte, dev);
+    rc = b200_fp8_blockwise_scaled_mm_splitk(xp, K, wp, K, xsp, xs_m, xs_g, wsp, ws_n, ws_g, out.data_ptr(), N, dt_of(ot), M,
+                                             N, K, 0, bytes ? work.data_ptr() : nullptr, bytes, stream_of(dev));
+  }
   if (rc != 0) return raise_status("w8a8_block_fp8_matmul", rc);
   return THPVariable_Wrap(std::move(out));
 }
@@ -285,13 +331,20 @@ HOST_FN(matmul_packed) {
   if (ws->size(0) != N / 128 || ws->size(1) != K / 128) return none();
   const at::Device dev = x->device();
   if (w->device() != dev || xs->device() != dev || ws->device() != dev) return none();
-  const c10::cuda::OptionalCUDAGuard guard(dev);
-  Tensor out = empty({M, N}, at::kBFloat16, dev);
   const bool pow2 = PyObject_IsTrue(a[4]);
-  const int rc = (pow2 ? b200_fp8_blockwise_scaled_mm_pow2 : b200_fp8_blockwise_scaled_mm_ue8m0)(
-      x->data_ptr(), K, w->data_ptr(), K, static_cast<const uint32_t*>(xs->data_ptr()), xs->stride(0), xs->stride(1),
-      static_cast<const float*>(ws->data_ptr()), ws->stride(0), ws->stride(1), out.data_ptr(), N, B200_DT_BF16, M, N, K,
-      stream_of(dev));
+  const void *xp = x->data_ptr(), *wp = w->data_ptr();
+  const uint32_t* xsp = static_cast<const uint32_t*>(xs->data_ptr());
+  const float* wsp = static_cast<const float*>(ws->data_ptr());
+  const int64_t xs_m = xs->stride(0), xs_g = xs->stride(1), ws_n = ws->stride(0), ws_g = ws->stride(1);
+  Tensor out;
+  int rc;
+  {
+    const NoGil no_gil;
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    out = empty({M, N}, at::kBFloat16, dev);
+    rc = (pow2 ? b200_fp8_blockwise_scaled_mm_pow2 : b200_fp8_blockwise_scaled_mm_ue8m0)(
+        xp, K, wp, K, xsp, xs_m, xs_g, wsp, ws_n, ws_g, out.data_ptr(), N, B200_DT_BF16, M, N, K, stream_of(dev));
+  }
   if (rc != 0) return raise_status("w8a8_block_fp8_matmul_deepgemm", rc);
   return THPVariable_Wrap(std::move(out));
 }
@@ -312,14 +365,22 @@ HOST_FN(gate_up_silu_quant) {
   if (xs->size(0) != M || xs->size(1) < (K / 128 + 3) / 4 || ws->size(0) != n2 / 128 || ws->size(1) != K / 128) return none();
   const at::Device dev = x->device();
   if (w->device() != dev || xs->device() != dev || ws->device() != dev) return none();
-  const c10::cuda::OptionalCUDAGuard guard(dev);
-  Tensor q = empty({M, N}, at::kFloat8_e4m3fn, dev);
-  int64_t rs, gs;
-  Tensor s = scale_tensor(*x, N, M, 128, true, true, true, true, dev, rs, gs);
-  const int rc = b200_fp8_gate_up_silu_quant_pow2(
-      x->data_ptr(), K, w->data_ptr(), K, static_cast<const uint32_t*>(xs->data_ptr()), xs->stride(0), xs->stride(1),
-      static_cast<const float*>(ws->data_ptr()), ws->stride(0), ws->stride(1), q.data_ptr(), N,
-      static_cast<uint32_t*>(s.data_ptr()), gs, dt_of(mid), M, N, K, stream_of(dev));
+  const auto sizes = x->sizes().vec();
+  const void *xp = x->data_ptr(), *wp = w->data_ptr();
+  const uint32_t* xsp = static_cast<const uint32_t*>(xs->data_ptr());
+  const float* wsp = static_cast<const float*>(ws->data_ptr());
+  const int64_t xs_m = xs->stride(0), xs_g = xs->stride(1), ws_n = ws->stride(0), ws_g = ws->stride(1);
+  Tensor q, s;
+  int rc;
+  {
+    const NoGil no_gil;
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    q = empty({M, N}, at::kFloat8_e4m3fn, dev);
+    int64_t rs, gs;
+    s = scale_tensor(sizes, N, M, 128, true, true, true, true, dev, rs, gs);
+    rc = b200_fp8_gate_up_silu_quant_pow2(xp, K, wp, K, xsp, xs_m, xs_g, wsp, ws_n, ws_g, q.data_ptr(), N,
+                                          static_cast<uint32_t*>(s.data_ptr()), gs, dt_of(mid), M, N, K, stream_of(dev));
+  }
   if (rc != 0) return raise_status("gate_up_silu_quant_pow2", rc);
   return pair_of(std::move(q), std::move(s));
 }
@@ -333,11 +394,19 @@ HOST_FN(topk_softmax) {
   const int64_t m = x->size(0), E = x->size(1), topk = PyLong_AsLong(a[1]);
   if (m == 0 || topk <= 0 || topk > E || topk > 32 || E > 1024 || x->stride(0) < E) return none();
   const at::Device dev = x->device();
-  const c10::cuda::OptionalCUDAGuard guard(dev);
-  Tensor w = empty({m, topk}, at::kFloat, dev), ids = empty({m, topk}, at::kInt, dev);
-  const int rc = b200_topk_softmax(x->data_ptr(), dt_of(x->scalar_type()), x->stride(0), static_cast<float*>(w.data_ptr()),
-                                   static_cast<int32_t*>(ids.data_ptr()), m, static_cast<int>(E), static_cast<int>(topk),
-                                   PyObject_IsTrue(a[2]) ? 1 : 0, stream_of(dev));
+  const int dt = dt_of(x->scalar_type()), renormalize = PyObject_IsTrue(a[2]) ? 1 : 0;
+  const int64_t ld = x->stride(0);
+  const void* xp = x->data_ptr();
+  Tensor w, ids;
+  int rc;
+  {
+    const NoGil no_gil;
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    w = empty({m, topk}, at::kFloat, dev);
+    ids = empty({m, topk}, at::kInt, dev);
+    rc = b200_topk_softmax(xp, dt, ld, static_cast<float*>(w.data_ptr()), static_cast<int32_t*>(ids.data_ptr()), m,
+                           static_cast<int>(E), static_cast<int>(topk), renormalize, stream_of(dev));
+  }
   if (rc != 0) return raise_status("topk_softmax", rc);
   return pair_of(std::move(w), std::move(ids));
 }
@@ -359,13 +428,20 @@ HOST_FN(fused_gate) {
       (shared > 0 && factor == 0.0) || x->stride(0) < E)
     return none();
   const at::Device dev = x->device();
-  const c10::cuda::OptionalCUDAGuard guard(dev);
-  Tensor w = empty({m, topk}, at::kFloat, dev), ids = empty({m, topk}, at::kInt, dev);
-  const int rc = b200_moe_fused_gate_shared_experts(
-      static_cast<const float*>(x->data_ptr()), x->stride(0), static_cast<const float*>(b->data_ptr()),
-      static_cast<float*>(w.data_ptr()), static_cast<int32_t*>(ids.data_ptr()), m, static_cast<int>(E),
-      static_cast<int>(groups), static_cast<int>(tg), static_cast<int>(topk), static_cast<int>(shared),
-      shared ? factor : 1.0, stream_of(dev));
+  const int64_t ld = x->stride(0);
+  const float *xp = static_cast<const float*>(x->data_ptr()), *bp = static_cast<const float*>(b->data_ptr());
+  Tensor w, ids;
+  int rc;
+  {
+    const NoGil no_gil;
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    w = empty({m, topk}, at::kFloat, dev);
+    ids = empty({m, topk}, at::kInt, dev);
+    rc = b200_moe_fused_gate_shared_experts(xp, ld, bp, static_cast<float*>(w.data_ptr()),
+                                            static_cast<int32_t*>(ids.data_ptr()), m, static_cast<int>(E),
+                                            static_cast<int>(groups), static_cast<int>(tg), static_cast<int>(topk),
+                                            static_cast<int>(shared), shared ? factor : 1.0, stream_of(dev));
+  }
   if (rc != 0) return raise_status("moe_fused_gate", rc);
   return pair_of(std::move(w), std::move(ids));
 }
@@ -400,15 +476,23 @@ HOST_FN(experts) {
     tables[i] = static_cast<int32_t*>(t->data_ptr());
   }
   const int ue8m0 = PyObject_IsTrue(a[10]) ? 1 : 0;
-  const c10::cuda::OptionalCUDAGuard guard(dev);
-  Tensor out = empty({m, k}, x->scalar_type(), dev);
-  const size_t bytes = b200_fused_experts_fp8_workspace_bytes(m, k, N, static_cast<int>(topk), static_cast<int>(E), ue8m0);
-  const Tensor work = empty({static_cast<int64_t>(bytes)}, at::kByte, dev);
-  const int rc = b200_fused_experts_fp8(
-      x->data_ptr(), dt_of(x->scalar_type()), w13->data_ptr(), w2->data_ptr(), static_cast<const float*>(s13->data_ptr()),
-      static_cast<const float*>(s2->data_ptr()), static_cast<const float*>(tw->data_ptr()),
-      static_cast<const int32_t*>(ti->data_ptr()), m, k, N, static_cast<int>(topk), static_cast<int>(E), tables[0],
-      tables[1], tables[2], out.data_ptr(), ue8m0, work.data_ptr(), bytes, stream_of(dev));
+  const at::ScalarType xt = x->scalar_type();
+  const void *xp = x->data_ptr(), *w13p = w13->data_ptr(), *w2p = w2->data_ptr();
+  const float *s13p = static_cast<const float*>(s13->data_ptr()), *s2p = static_cast<const float*>(s2->data_ptr()),
+              *twp = static_cast<const float*>(tw->data_ptr());
+  const int32_t* tip = static_cast<const int32_t*>(ti->data_ptr());
+  Tensor out;
+  int rc;
+  {
+    const NoGil no_gil;
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    out = empty({m, k}, xt, dev);
+    const size_t bytes = b200_fused_experts_fp8_workspace_bytes(m, k, N, static_cast<int>(topk), static_cast<int>(E), ue8m0);
+    const Tensor work = empty({static_cast<int64_t>(bytes)}, at::kByte, dev);
+    rc = b200_fused_experts_fp8(xp, dt_of(xt), w13p, w2p, s13p, s2p, twp, tip, m, k, N, static_cast<int>(topk),
+                                static_cast<int>(E), tables[0], tables[1], tables[2], out.data_ptr(), ue8m0,
+                                work.data_ptr(), bytes, stream_of(dev));
+  }
   if (rc != 0) return raise_status("fused_experts_fp8", rc);
   return THPVariable_Wrap(std::move(out));
 }
