@@ -12,6 +12,7 @@
 #include <ATen/EmptyTensor.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/DynamicTypes.h>
@@ -97,7 +98,7 @@ Tensor scale_tensor(std::vector<int64_t> sizes, int64_t K, int64_t M, int64_t gr
     gs = ld;
     Tensor whole = empty({W, ld}, at::kInt, dev);
     if (ld != M || (partial && G % 4 != 0))
-      (void)cudaMemsetAsync(whole.data_ptr(), 0, W * ld * 4, static_cast<cudaStream_t>(stream_of(dev)));
+      C10_CUDA_CHECK(cudaMemsetAsync(whole.data_ptr(), 0, W * ld * 4, static_cast<cudaStream_t>(stream_of(dev))));
     return whole.transpose(0, 1).narrow(0, 0, M);
   }
   if (col_major) {      // 2-D only (checked by the callers)
