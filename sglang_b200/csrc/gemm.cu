@@ -508,8 +508,7 @@ int launch_reduce(const GemmParams& p, cudaStream_t stream) {
   int64_t blocks = (total + 255) / 256;
   if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
   launch_pdl(splitk_reduce_kernel<OutT>, static_cast<int>(blocks), 256, 0, stream, p.partial, static_cast<OutT*>(p.out),
-             static_cast<const OutT*>(p.bias), p.M, p.N,
-                                                                         p.ldo, p.split_k);
+             static_cast<const OutT*>(p.bias), p.M, p.N, p.ldo, p.split_k);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
 }
@@ -557,8 +556,7 @@ int launch_tail_reduce(const GemmParams& p, cudaStream_t stream) {
   const int n_blocks = (p.N + p.tile_n - 1) / p.tile_n;
   const dim3 grid(m_blocks * n_blocks - p.tail_first, kTailSlices);
   launch_pdl(tail_reduce_kernel<OutT>, grid, 256, 0, stream, p.partial, static_cast<OutT*>(p.out),
-             static_cast<const OutT*>(p.bias), p.M, p.N, p.ldo, p.split_k,
-                                                     p.tail_first, m_blocks, n_blocks, p.tile_n);
+             static_cast<const OutT*>(p.bias), p.M, p.N, p.ldo, p.split_k, p.tail_first, m_blocks, n_blocks, p.tile_n);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
 }
@@ -621,9 +619,6 @@ inline int forced_token_tile() {
   return g_force_block_n == 3032 ? 32 : g_force_block_n == 3064 ? 64 : g_force_block_n == 3128 ? 128 : 0;
 }
 
-}  // namespace b200
-
-namespace b200 {
 namespace {
 
 // Which kernel a dense problem gets.  Up to 64 tokens the weight-streaming kernel (gemm_swapab.cu, 128 weight rows x up to

@@ -59,12 +59,10 @@ int bias_add(void* out, const void* bias, int64_t M, int64_t N, int64_t ldo, int
   const int64_t blocks = std::min<int64_t>((M * (N / 2) + 255) / 256, 16LL * sm_count());
   if (dtype == B200_DT_BF16)
     launch_pdl(bias_add_kernel<__nv_bfloat16>, static_cast<unsigned>(blocks), 256, 0, st, static_cast<__nv_bfloat16*>(out),
-                                                                   static_cast<const __nv_bfloat16*>(bias), M,
-                                                                   static_cast<int>(N), ldo);
+               static_cast<const __nv_bfloat16*>(bias), M, static_cast<int>(N), ldo);
   else
     launch_pdl(bias_add_kernel<__half>, static_cast<unsigned>(blocks), 256, 0, st, static_cast<__half*>(out),
-                                                                   static_cast<const __half*>(bias), M,
-                                                                   static_cast<int>(N), ldo);
+               static_cast<const __half*>(bias), M, static_cast<int>(N), ldo);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
 }

@@ -310,7 +310,7 @@ silu_and_mul_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t rows, 
 template <typename T, typename F>
 __global__ void __launch_bounds__(256)
 unpermute_sum_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __restrict__ perm,
-                     const F* __restrict__ factors, int m, int topk, int row_len) {
+                     const F* __restrict__ factors, int topk, int row_len) {
   pdl_start();
   const int vec_per_row = row_len / 8, parts = (vec_per_row + blockDim.x - 1) / blockDim.x;
   const int i = blockIdx.x / parts, v = (blockIdx.x - i * parts) * blockDim.x + threadIdx.x;
@@ -368,14 +368,14 @@ int moe_prepare_launch(const int32_t* topk_ids, int64_t n_ids, int topk, int num
   }
   launch_pdl(prep_count_kernel, nch, kPrepThreads, num_experts * sizeof(int32_t), st, topk_ids, n_ids, num_experts, scratch);
   launch_pdl(prep_scan_kernel, 1, 1024, num_experts * sizeof(int32_t), st, scratch, nch, num_experts, expert_offsets,
-                                                                   blockscale_offsets, problem_sizes1,
-                                                                   problem_sizes2, n, k);
+             blockscale_offsets, problem_sizes1, problem_sizes2, n, k);
   // walking warps: as many (a power of two up to 8) as fit their per-expert tables into 48 KB of shared memory
   int walk_warps = 8;
   while (walk_warps > 1 && (static_cast<size_t>(walk_warps) * num_experts + kPrepChunk) * sizeof(int32_t) > 48 * 1024)
     walk_warps >>= 1;
-  launch_pdl(prep_scatter_kernel, nch, kPrepThreads, (static_cast<size_t>(walk_warps) * num_experts + kPrepChunk) * sizeof(int32_t), st, 
-      topk_ids, n_ids, topk, num_experts, scratch, input_permutation, output_permutation, walk_warps);
+  launch_pdl(prep_scatter_kernel, nch, kPrepThreads,
+             (static_cast<size_t>(walk_warps) * num_experts + kPrepChunk) * sizeof(int32_t), st, topk_ids, n_ids, topk,
+             num_experts, scratch, input_permutation, output_permutation, walk_warps);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
 }
@@ -489,8 +489,8 @@ extern "C" int b200_shuffle_packed_scales(const uint32_t* input, int64_t input_s
   const int64_t blocks = (num_dst_rows + 255) / 256;
   if (blocks > 0x7fffffffLL || words_per_row > 65535) return B200_ERR_TOO_LARGE;
   launch_pdl(packed_scales_gather_kernel, dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(words_per_row)), 256, 0,
-                                static_cast<cudaStream_t>(stream), input, input_stride_pack, num_src_rows, dst2src_map,
-                                                                     output, output_stride_pack, num_dst_rows);
+             static_cast<cudaStream_t>(stream), input, input_stride_pack, num_src_rows, dst2src_map, output,
+             output_stride_pack, num_dst_rows);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
 }
@@ -511,20 +511,16 @@ extern "C" int b200_shuffle_rows(const void* input, const int32_t* dst2src_map, 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if ((bits & 15u) == 0) {
     launch_pdl(rows_gather_kernel<uint4>, grid, 256, 0, st, static_cast<const uint4*>(input), dst2src_map,
-                                                    static_cast<uint4*>(output), num_dst_rows,
-                                                    static_cast<int>(row_bytes / 16));
+               static_cast<uint4*>(output), num_dst_rows, static_cast<int>(row_bytes / 16));
   } else if ((bits & 7u) == 0) {
     launch_pdl(rows_gather_kernel<uint2>, grid, 256, 0, st, static_cast<const uint2*>(input), dst2src_map,
-                                                    static_cast<uint2*>(output), num_dst_rows,
-                                                    static_cast<int>(row_bytes / 8));
+               static_cast<uint2*>(output), num_dst_rows, static_cast<int>(row_bytes / 8));
   } else if ((bits & 3u) == 0) {
     launch_pdl(rows_gather_kernel<uint32_t>, grid, 256, 0, st, static_cast<const uint32_t*>(input), dst2src_map,
-                                                       static_cast<uint32_t*>(output), num_dst_rows,
-                                                       static_cast<int>(row_bytes / 4));
+               static_cast<uint32_t*>(output), num_dst_rows, static_cast<int>(row_bytes / 4));
   } else {
     launch_pdl(rows_gather_kernel<uint8_t>, grid, 256, 0, st, static_cast<const uint8_t*>(input), dst2src_map,
-                                                      static_cast<uint8_t*>(output), num_dst_rows,
-                                                      static_cast<int>(row_bytes));
+               static_cast<uint8_t*>(output), num_dst_rows, static_cast<int>(row_bytes));
   }
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
@@ -542,11 +538,11 @@ extern "C" int b200_silu_and_mul(const void* x, void* out, int64_t rows, int64_t
   if (blocks > cap) blocks = cap;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == B200_DT_BF16) {
-    launch_pdl(silu_and_mul_kernel<__nv_bfloat16>, static_cast<unsigned>(blocks), 256, 0, st, 
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out), rows, static_cast<int>(d));
+    launch_pdl(silu_and_mul_kernel<__nv_bfloat16>, static_cast<unsigned>(blocks), 256, 0, st, static_cast<const __nv_bfloat16*>(x),
+               static_cast<__nv_bfloat16*>(out), rows, static_cast<int>(d));
   } else if (dtype == B200_DT_F16) {
-    launch_pdl(silu_and_mul_kernel<__half>, static_cast<unsigned>(blocks), 256, 0, st, 
-        static_cast<const __half*>(x), static_cast<__half*>(out), rows, static_cast<int>(d));
+    launch_pdl(silu_and_mul_kernel<__half>, static_cast<unsigned>(blocks), 256, 0, st, static_cast<const __half*>(x),
+               static_cast<__half*>(out), rows, static_cast<int>(d));
   } else {
     return B200_ERR_BAD_DTYPE;
   }
@@ -571,9 +567,8 @@ int unpermute_sum(const void* input, void* output, const int32_t* permutation, c
   auto go = [&](auto* in) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(in)>>;
     using Factor = std::conditional_t<std::is_void_v<F>, T, F>;
-    launch_pdl(unpermute_sum_kernel<T, Factor>, static_cast<unsigned>(blocks), threads, 0, st, in,
-        static_cast<T*>(output), permutation, static_cast<const Factor*>(factors), static_cast<int>(m),
-        static_cast<int>(topk), static_cast<int>(row_len));
+    launch_pdl(unpermute_sum_kernel<T, Factor>, static_cast<unsigned>(blocks), threads, 0, st, in, static_cast<T*>(output),
+               permutation, static_cast<const Factor*>(factors), static_cast<int>(topk), static_cast<int>(row_len));
   };
   if (dtype == B200_DT_BF16) go(static_cast<const __nv_bfloat16*>(input));
   else if (dtype == B200_DT_F16) go(static_cast<const __half*>(input));
@@ -875,12 +870,10 @@ extern "C" int b200_moe_fused_gate_shared_experts(const float* gating_output, in
   const size_t smem = 4 * static_cast<size_t>(num_experts) * sizeof(float);
   if (num_experts <= 256)
     launch_pdl(fused_gate_kernel<8>, blocks, 128, smem, st, gating_output, bias, topk_weights, topk_ids, num_tokens, num_experts,
-                                                   num_expert_group, topk_group, topk, row_stride,
-                                                   num_fused_shared_experts, routed_scaling_factor);
+               num_expert_group, topk_group, topk, row_stride, num_fused_shared_experts, routed_scaling_factor);
   else
     launch_pdl(fused_gate_kernel<32>, blocks, 128, smem, st, gating_output, bias, topk_weights, topk_ids, num_tokens, num_experts,
-                                                    num_expert_group, topk_group, topk, row_stride,
-                                                    num_fused_shared_experts, routed_scaling_factor);
+               num_expert_group, topk_group, topk, row_stride, num_fused_shared_experts, routed_scaling_factor);
   B200_CUDA_TRY(cudaGetLastError());
   return B200_OK;
 }

@@ -504,9 +504,9 @@ int launch_group(const void* x, void* q, float* s, int64_t M, int64_t K, int64_t
   const dim3 grid(static_cast<unsigned>(tiles));
   const T* xp = static_cast<const T*>(x);
   uint8_t* qp = static_cast<uint8_t*>(q);
-#define B200_LAUNCH_Q(P)                                                                                       \
-  launch_pdl(quant_group_kernel<T, GROUP, P, IEEE_DIV, FUSE_SILU, UE8M0, INT8>, grid, kThreads, 0, stream, xp, src_rows, x_rows, qp, s, M, K, ssr, ssg, eps, fmin_, \
-                                                                           fmax_, tiles_k)
+#define B200_LAUNCH_Q(P)                                                                                              \
+  launch_pdl(quant_group_kernel<T, GROUP, P, IEEE_DIV, FUSE_SILU, UE8M0, INT8>, grid, kThreads, 0, stream, xp, src_rows, \
+             x_rows, qp, s, M, K, ssr, ssg, eps, fmin_, fmax_, tiles_k)
   switch (passes) {
     case 8:
       if constexpr (kMaxPasses >= 8) { B200_LAUNCH_Q(8); }
@@ -750,10 +750,9 @@ extern "C" int b200_rmsnorm_per_token_group_quant_fp8(const void* x, int x_dtype
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const dim3 grid(static_cast<unsigned>(M));
 #define B200_NORM_GO(T, NV, WQ, UE, RES)                                                                              \
-  launch_pdl(rmsnorm_quant_kernel<T, WQ, UE, NV, RES>, grid, kThreads, 0, st, \
-      static_cast<const T*>(x), static_cast<T*>(residual), static_cast<const T*>(weight), static_cast<T*>(y),         \
-      static_cast<uint8_t*>(q), static_cast<float*>(s), M, K, s_stride_row, s_stride_grp, norm_eps, eps, fp8_min,     \
-      fp8_max)
+  launch_pdl(rmsnorm_quant_kernel<T, WQ, UE, NV, RES>, grid, kThreads, 0, st, static_cast<const T*>(x),               \
+             static_cast<T*>(residual), static_cast<const T*>(weight), static_cast<T*>(y), static_cast<uint8_t*>(q),  \
+             static_cast<float*>(s), M, K, s_stride_row, s_stride_grp, norm_eps, eps, fp8_min, fp8_max)
 #define B200_NORM_NV(T, NV)                                       \
   do {                                                            \
     if (residual) {                                               \
