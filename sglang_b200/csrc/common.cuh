@@ -213,14 +213,22 @@ __device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded by a count of tries (a failed try suspends the thread in hardware for a while, so the limit is seconds): no
-// clock reads and one register in the loop.
-constexpr uint32_t kWaitTries = 1u << 26;
+// Bounded like mbar_wait: by the SM clock, and by the launch's status word.  Both are looked at once in 256 tries, the
+// clock in units of 2^20 cycles, so that the loop holds two registers and a wait that ends soon reads neither.
+constexpr uint32_t kWaitLimitUnits = static_cast<uint32_t>(kWaitLimitCycles >> 20);
 __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, int* status, int code) {
-  for (uint32_t n = 0; n < kWaitTries; ++n)
-    if (try_wait(bar, parity)) return true;
-  report_wait_failure(status, code);
-  return false;
+  uint32_t t0 = 0;
+  for (uint32_t n = 1; !try_wait(bar, parity); ++n) {
+    if ((n & 0xffu) != 0) continue;
+    const uint32_t now = static_cast<uint32_t>(clock64() >> 20);
+    if (n == 256) t0 = now;
+    if (*reinterpret_cast<volatile int*>(status) != 0) return false;   // another wait of this launch gave up
+    if (now - t0 > kWaitLimitUnits) {
+      report_wait_failure(status, code);
+      return false;
+    }
+  }
+  return true;
 }
 __device__ __forceinline__ void arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
