@@ -83,6 +83,19 @@ __device__ __forceinline__ void pdl_start() {
   pdl_wait();
   pdl_trigger();
 }
+// For roles that begin with a bounded mbarrier wait: the wait must not start while an earlier kernel, of whatever length,
+// holds this one up.  One warp does pdl_wait and then calls pdl_release; the others block in pdl_await_release (named
+// barrier 1, THREADS = both sides' threads).  A pdl_wait in each warp instead measured 2 % slower on decode linears
+// (1 x 8192 x 8192 17.05 against 16.70 us, 16 x 7168 x 18432 28.9 against 28.4).
+template <int THREADS>
+__device__ __forceinline__ void pdl_release() {
+  __syncwarp();
+  asm volatile("bar.arrive 1, %0;" ::"n"(THREADS) : "memory");
+}
+template <int THREADS>
+__device__ __forceinline__ void pdl_await_release() {
+  asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+}
 
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;

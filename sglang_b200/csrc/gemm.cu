@@ -53,6 +53,7 @@ constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kEpiWarps = 8;
 constexpr int kTmaWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1, kStagerWarp = kEpiWarps + 2;
 constexpr int kThreads = 32 * (kEpiWarps + 4);
+constexpr int kReleaseThreads = 32 * (kEpiWarps + 2);   // TMA warp, MMA warp, read-out warps (pdl_release)
 constexpr int CPW = 128;        // columns per read-out warp: one half of the tile
 constexpr int kChunk = 64;      // columns per tensor-memory round trip (32: up to 4 % slower from 512 rows on)
 constexpr int kSlotFloats = TILE_M * kScaleGroup + 2 * kScaleGroup;   // [128 rows][4 k-blocks], then [2 halves][4]
@@ -225,6 +226,7 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         __syncwarp();
       }
       pdl_wait();
+      pdl_release<kReleaseThreads>();
     }
     pdl_trigger_if(num_vtiles <= static_cast<int>(gridDim.x));
     for (int vt = blockIdx.x; ok && vt < num_vtiles; vt += gridDim.x) {
@@ -256,6 +258,7 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------------ MMA issuer
     // The whole warp walks the loop so that addresses and descriptors stay warp-uniform; one elected lane issues.
+    if constexpr (!GROUPED) pdl_await_release<kReleaseThreads>();
     const uint64_t a_desc0 = umma_desc_k128(smem_a);
     const uint64_t b_desc0 = umma_desc_k128(smem_b);
     int stage = 0;
@@ -343,6 +346,7 @@ gemm_block_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   } else {
     // ====================================================================== promotion + epilogue warps
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
+    if constexpr (!GROUPED) pdl_await_release<kReleaseThreads>();
     // What the loop below needs is worked out again from the parameter block and the special registers: values computed
     // before the branch stay live next to 128 accumulators, and ptxas then spills (to a local memory with almost no L1).
     int m_blocks, n_blocks, nkb, num_vtiles, split_k, warp, lane;

@@ -29,6 +29,7 @@ constexpr int kPair = 2;         // k-blocks per pipeline stage and per hand-off
 constexpr int kScaleGroup = 8;   // k-blocks per scale-ring slot (8 fp32 scales of a token = one 32-byte sector)
 constexpr int kScaleSlots = 4;
 constexpr int kEpiWarps = 8;     // 4 lane quadrants x 2 column halves
+constexpr int kReleaseThreads = 32 * (kEpiWarps + 2);   // TMA warp, MMA warp, read-out warps (pdl_release)
 constexpr int kMaxExperts = 1024;
 
 template <int TN>
@@ -209,6 +210,7 @@ gemm_block_fp8_swapab_kernel(const __grid_constant__ CUtensorMap map_w, const __
         __syncwarp();
       }
       pdl_wait();
+      pdl_release<kReleaseThreads>();
     }
     pdl_trigger_if(num_vtiles <= static_cast<int>(gridDim.x));
     for (int vt = blockIdx.x; ok && vt < num_vtiles; vt += gridDim.x) {
@@ -240,6 +242,7 @@ gemm_block_fp8_swapab_kernel(const __grid_constant__ CUtensorMap map_w, const __
     // D[weight row, token] = W_tile (128 x 128 B, the instruction's M side) x X_tile^T (tn tokens, its
     // N side); tn = tokens of the tile rounded up to 16, encoded in the instruction descriptor.  The two
     // k-blocks of a stage go to the two accumulators of a pair; one commit covers both.
+    if constexpr (!GROUPED) pdl_await_release<kReleaseThreads>();
     const uint64_t w_desc0 = umma_desc_k128(smem_u32(smem_w));
     const uint64_t x_desc0 = umma_desc_k128(smem_u32(smem_x));
     int stage = 0, ap = 0;
@@ -351,6 +354,7 @@ gemm_block_fp8_swapab_kernel(const __grid_constant__ CUtensorMap map_w, const __
   } else {
     // ====================================================================== promotion + epilogue warps
     if constexpr (C::kRebalanceRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kEpiRegs));
+    if constexpr (!GROUPED) pdl_await_release<kReleaseThreads>();
     // The accumulator is read in the 16-lane fragment layout (tcgen05.ld 16x256b): a thread then holds
     // 4 weight rows x CPW/4 tokens instead of 1 row x CPW tokens, so it needs only CPW/4 scale products
     // per k-block.  (With one row per thread every thread reads every token's product, and the

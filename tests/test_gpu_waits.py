@@ -1,10 +1,12 @@
-"""GPU: the bounded waits end where they say."""
+"""GPU: the bounded waits end where they say, and time spent behind another kernel does not count against them."""
 import ctypes
 import os
 import subprocess
 
 import pytest
 import torch
+
+from oracle import block_fp8_oracle as O
 
 pytestmark = pytest.mark.gpu
 LIMIT = 2_000_000_000       # cycles, kWaitLimitCycles
@@ -20,6 +22,7 @@ def probe(tmp_path_factory):
                    capture_output=True)
     lib = ctypes.CDLL(so)
     lib.probe_wait_out.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    lib.probe_early_trigger.argtypes = [ctypes.c_longlong, ctypes.c_void_p]
     return lib
 
 
@@ -48,3 +51,30 @@ def test_a_wait_leaves_when_another_wait_of_its_launch_gave_up(probe, form):
     returned, cycles, slot, sticky = _wait_out(probe, form, 5)
     assert (returned, slot, sticky) == (0, 5, 0)        # nothing is reported twice
     assert cycles < 0.25 * LIMIT, cycles
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 1024, 1024), (256, 1024, 1024), (1024, 1024, 1024)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_a_busy_predecessor_is_not_a_timeout(probe, M, N, K, packed):
+    """A kernel that lets its dependents start and then runs for longer than a wait's limit: the GEMM behind it gives its
+    usual result."""
+    from sglang_b200 import _lib
+    from sglang_b200.layers.quantization.fp8_kernel import (sglang_per_token_group_quant_fp8, w8a8_block_fp8_matmul,
+                                                            w8a8_block_fp8_matmul_deepgemm)
+    x = torch.randn(M, K, generator=torch.Generator(device="cuda").manual_seed(M), device="cuda").to(torch.bfloat16)
+    w, s = O.per_block_quant_mxfp8(torch.randn(N, K, generator=torch.Generator().manual_seed(N)) * 0.02)
+    w, s = w.cuda(), s.cuda()
+    if packed:
+        q, qs = sglang_per_token_group_quant_fp8(x, 128, column_major_scales=True, scale_tma_aligned=True, scale_ue8m0=True)
+        call = lambda: w8a8_block_fp8_matmul_deepgemm(q, w, qs, s, [128, 128], torch.bfloat16, weight_scale_ue8m0=True)
+    else:
+        q, qs = sglang_per_token_group_quant_fp8(x, 128)
+        call = lambda: w8a8_block_fp8_matmul(q, w, qs, s, [128, 128], torch.bfloat16)
+    usual = call()
+    torch.cuda.synchronize()
+    assert probe.probe_early_trigger(LIMIT + LIMIT // 2, torch.cuda.current_stream().cuda_stream) == 0
+    behind = call()
+    status = ctypes.c_int(0)
+    _lib.check("status", _lib.lib().b200_gemm_device_status(ctypes.byref(status)))
+    assert status.value == 0
+    assert torch.equal(behind, usual)
