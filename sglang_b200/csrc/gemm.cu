@@ -26,9 +26,10 @@
 //   * spill: shared memory takes the whole L1, so a spilled register is an L2 round trip.  Eight warps of 128 columns with
 //     216 registers hold the accumulators and a 64-column chunk; sixteen warps of 64 columns (104 registers) spill;
 //   * write its row in 16-byte pieces (863 -> 803 with 32-byte stores).
-// What bounds it now at large M is power: 803 cycles at the 1.45-1.5 GHz that the chip holds, where the same loop without
-// stores runs 739.  (A CTA pair with two 128-column halves and four accumulators measured 946 cycles without loads or
-// scales: the accumulator's round trip crosses the cluster.)
+// What bounds it now is the chain of waits in the read-out warps: 803 cycles per k-block (739 without the stores) where the
+// MMAs need 512, as many on zeros as on random data.  Power only sets the clock that they run at: at large M 1.45 GHz on
+// random data and 1.965 GHz on zeros (1050 and 784 us for the product above).  (A CTA pair with two 128-column halves and
+// four accumulators measured 946 cycles without loads or scales: the accumulator's round trip crosses the cluster.)
 // All mbarrier waits are bounded; a wait that gives up records a code in a device status word and every role drains to
 // a common exit where tensor memory is released.
 #include <algorithm>
@@ -745,13 +746,17 @@ DensePlan plan_dense(int64_t M, int64_t N, int64_t K, int sms, bool swapab, size
 
 // A linear with power-of-two scales on both operands: whether the promoting kernels of this file and gemm_swapab.cu take the
 // product (exponent bytes decoded to fp32 scales) instead of the block-scaling one, which accumulates in tensor memory
-// without read-outs but cannot divide a tile's k-blocks.  us, promoting / block-scaling:
-//   few tiles: 16 x 7168 x 18432 27 / 46, 128 x 8192 x 8192 19.1 / 24.2, 256 x 1280 x 8192 16.0 / 22.9
-//   its 128 x 128 tiles fill more than half of the SMs once: 128 x 10240 x 8192 29.0 / 26.4, 256 x 8192 x 8192 28.2 / 24.7,
-//     512 x 4096 x 7168 25.0 / 22.1 -- up to 64 rows the weight-streaming kernel is still ahead (64 x 10240 x 8192
-//     21.7 / 25.0), and so are its splits at very long K (256 x 8192 x 28672 71.8 / 78.8)
-//   more than one such wave: 640 x 57344 x 8192 295 / 350, 768 x 7168 x 18432 101 / 139, 768 x 36864 x 7168 184 / 178
-//   from 1024 rows on: 1024 x 7168 x 18432 143 / 115, 2048 x 8192 x 8192 140 / 129
+// without read-outs but cannot divide a tile's k-blocks.  us with the quantiser, promoting / block-scaling:
+//   few tiles: 16 x 7168 x 18432 28 / 49, 128 x 8192 x 8192 22 / 27, 256 x 1280 x 8192 18 / 26
+//   up to 64 rows: 64 x 10240 x 8192 25.4 / 27.3, 64 x 18432 x 7168 28.3 / 30.3
+//   its 128 x 128 tiles fill more than half of the SMs once: below K = 16384 the two are within 6 % of each other
+//     (128 x 10240 x 12288 42.0 / 39.3, 256 x 8192 x 14336 48.8 / 46.8, 256 x 7168 x 8192 28.3 / 29.1) but for nearly full
+//     waves, whose tiles leave no SMs to divide k-blocks over (128 x 18432 x 14336 66 / 54); above it the splits lead
+//     (512 x 4096 x 16384 50.8 / 52.5, 256 x 7168 x 18432 54.6 / 56.5, 128 x 10240 x 28672 71 / 83), again but for nearly
+//     full waves, where this rule gives 7-15 % away (128 x 18432 x 16384 72 / 63, x 28672 107 / 100)
+//   more than one such wave: 640 x 57344 x 8192 281 / 317, 768 x 7168 x 18432 105 / 150, 320 x 36864 x 7168 96 / 103;
+//     on wide outputs the lead is gone by 768 rows (768 x 36864 x 7168 185 / 183, 1023 x 36864 x 7168 243 / 237)
+//   from 1024 rows on: 1024 x 7168 x 18432 141 / 128, 2048 x 8192 x 8192 135 / 131
 bool packed_promotes(int64_t M, int64_t N, int64_t K) {
   const int64_t tiles = ((M + 127) / 128) * ((N + 127) / 128);
   const bool one_full_wave = tiles <= sm_count() && 2 * tiles > sm_count();
