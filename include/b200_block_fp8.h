@@ -439,7 +439,9 @@ int b200_topk_softmax(const void* gating_output, int dtype, int64_t row_stride, 
  * One block-FP8 linear, start to finish: out[M,N] = quantise(x)[M,K] * w[N,K]^T (+ bias), the call sequence of
  * Fp8LinearMethod.apply (python/sglang/srt/layers/quantization/fp8.py:441-488).  x, bias [N] (or NULL) and out share
  * `dtype` (bf16 / fp16); bias is added to the rounded product.  K % 128 == 0.
- * scale_mode 0: fp32 scales; 1: power-of-two activation scales; 2: weight scales are powers of two as well.
+ * scale_mode 0: fp32 scales; 1: power-of-two activation scales; 2: weight scales are powers of two as well (the product
+ * then runs on b200_fp8_blockwise_scaled_mm_pow2 or, with fewer than 1024 rows, mostly on the fp32-promoting kernels,
+ * which can divide k-blocks among SMs: the same result up to the order of the fp32 additions).
  * Everything in between lives in `workspace` (b200_fp8_linear_workspace_bytes bytes, 16-byte aligned), which may be
  * reused by the next call on the same stream.  b200_sm_count: SMs the persistent kernels use on the current device
  * (its SMs, or the limit of b200_set_sm_limit).

@@ -111,7 +111,10 @@ def deepgemm_w8a8_block_fp8_linear_with_fallback(input: torch.Tensor, weight: to
     block-scaled product, bias, view back.  Shapes or dtypes the DeepGEMM path does not take fall back to
     the fp32-scale linear, as the reference falls back to its Triton kernel.  weight_scale_ue8m0=True promises
     power-of-two weight scales too (requant_weight_ue8m0): the product then runs on the tensor core's
-    block-scaling path, all k-blocks accumulated in tensor memory."""
+    block-scaling path, all k-blocks accumulated in tensor memory, from 1024 rows on and wherever its tiles
+    fill the GPU; fewer rows run on the fp32-promoting kernels, which can divide k-blocks among SMs.  The result
+    of a row can therefore differ with the number of rows by the order of the fp32 sums (an occasional last
+    bit of bf16).  SPLIT_K_MODE = "off" runs the block-scaling path, unsplit, at every size."""
     assert input_scale is None
     if gemm.SPLIT_K_MODE == "auto" and scale_ue8m0 and list(block_size) == [128, 128]:
         done = _lib.host().linear(input, weight, weight_scale, bias, None, 2 if weight_scale_ue8m0 else 1)
